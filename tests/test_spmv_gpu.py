@@ -345,3 +345,32 @@ def test_spmv_fast_short_rows_mode_within_plain_bound():
     assert np.all(np.abs(y[short] - ref[short]) <= plain[short] + 1e-30)
     assert_spmv_close(y[~short], ref[~short], scale[~short], lens[~short], "float32", "long rows")
     plan.set_fast_short_rows(False)
+
+
+@pytest.mark.parametrize("dname", DTYPES)
+@pytest.mark.parametrize("idx_dt", [torch.int32, torch.int64])
+@pytest.mark.parametrize("skip", [0, 1, 6])
+def test_spmv_row_blocks_run_edges(dname, idx_dt, skip):
+    """Row-block passes (runs of 4 or 2 nonzeros per lane): rows that end on, before and after
+    the ends of runs and passes, empty rows between and around them, rows at the window, arrays
+    that start off the wide loads' boundaries; and one infinite x entry stays in its own rows."""
+    lens = ([0, 1, 0, 2, 3, 4, 5] + [1] * 9 + [63, 64, 65, 0, 127, 128, 129, 0, 0, 223, 224, 225, 1, 0, 31, 33]
+            + [7] * 40 + [0] * 300 + [128, 128, 96, 32, 2] + [0, 3] * 50 + [1])
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz, k = int(ptr[-1]), 700
+    rng = np.random.Generator(np.random.PCG64(skip))
+    idx = rng.integers(0, k - 1, nnz).astype(np.int64)
+    hit = np.nonzero(np.asarray(lens) == 4)[0][0]
+    idx[ptr[hit]] = k - 1  # the only use of the last column
+    cplx = dname.startswith("complex")
+    data = rng.uniform(0.5, 1, nnz) + (1j * rng.uniform(0.5, 1, nnz) if cplx else 0)
+    x = rng.uniform(-1, 1, k) + (1j * rng.uniform(-1, 1, k) if cplx else 0)
+    dt = TORCH_DT[dname]
+    d = torch.cat([torch.zeros(skip, dtype=dt, device="cuda"), dev(data, dt)])[skip:]
+    i = torch.cat([torch.zeros(skip, dtype=idx_dt, device="cuda"), dev(idx, idx_dt)])[skip:]
+    p = fs.prepare_spmv_csr(d, i, dev(ptr), (len(lens), k))
+    y = fs.flagsparse_spmv_csr(x=dev(x, dt), prepared=p)
+    _check_against_oracle(y, ptr, idx, rounded(data, dname), rounded(x, dname), (len(lens), k), "non", dname, "edges")
+    x[-1] = np.inf
+    bad = ~np.isfinite(host(fs.flagsparse_spmv_csr(x=dev(x, dt), prepared=p)))
+    assert np.array_equal(np.nonzero(bad)[0], [hit])
