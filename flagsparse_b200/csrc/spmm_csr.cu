@@ -1,28 +1,19 @@
 // CSR SpMM  C = A B  for sm_100a (A sparse M x K in CSR, B dense K x N row-major).
 //
 // The launch reuses the SpMV unit plan (plan.cu), built with the SpMM window
-// cap (64) and chunk (256): every warp executes one (unit, column tile) pair.
-// The lanes of a warp own consecutive column groups of V elements of the tile
-// (16-byte loads when N and the leading dimensions allow it), so one nonzero
-// costs the warp a single coalesced read of its B-row slice:
-//
-//  * row-block unit: a run of rows with < 128 nonzeros.  The warp stages the
-//    nonzeros (value, column, local row) in its shared-memory slice, writes
-//    zero rows for empty rows, then walks the nonzeros in order, loading the
-//    B slices of 4 nonzeros ahead of the multiply-adds across row boundaries
-//    and storing a C row slice whenever the row changes.
-//  * long-row chunk: `chunk_nnz` nonzeros of a row with > cap nonzeros, staged
-//    in 128-nonzero batches.  A one-chunk row is written directly; otherwise
-//    the chunk's partial row slice goes to its scratch slot and the warp that
-//    completes the row's ticket adds the partials in chunk order.
+// cap (64) and chunk (256).  One kernel, k_spmm_team, serves every width: teams
+// of lanes own a column tile of B and C and take equal shares of the nonzeros
+// of a run of rows; long rows run as chunks whose partials are joined in order.
+// Rows of whole aligned 16-byte slices give each lane one slice; other widths
+// give it up to four smaller pieces (Slice).
 //
 // Accumulation: fp32 for half / bfloat16 / fp32 values (half and bfloat16
 // products are exact in fp32), fp64 for fp64, componentwise for complex.
 // FSB_SPMM_COMPENSATED switches every sum to Dot2 compensated accumulation.
 // Every sum runs in a fixed order, so results are bitwise reproducible.
 //
-// The same file holds the narrow-row team kernel (k_spmm_team, also fused
-// with an SpMV for the batched step) and the one-launch backward of Y = A X
+// The same file holds that kernel fused with an SpMV (the batched step) and
+// the one-launch backward of Y = A X
 // (k_spmm_bwd: dX = A^T dY and the SDDMM dvals from one gather of dY).
 //
 // Replaces _triton_spmm_csr_impl / _spmm_csr_real_kernel / the complex kernel
@@ -42,12 +33,6 @@ constexpr int kSpmmWarps = 8;      // warps per block; one (unit, tile) per warp
 constexpr int kSpmmBatch = 128;    // nonzeros staged per batch
 constexpr int kSpmmMaxCap = 64;    // row blocks hold < 2*cap <= kSpmmBatch nonzeros
 constexpr int kSpmmAhead = 4;      // B slices loaded ahead of the multiply-adds
-// the same for a team's row in the narrow-row kernel: 8 for fp32 (measured
-// 2-6 % faster), 4 where the slices, sums or the fused y terms need the registers
-template <int DT>
-struct TeamAhead { static constexpr int value = (DT == FSB_F32) ? 8 : 4; };
-constexpr int kSpmmTileLanes = 32;
-
 template <int BYTES> struct RawT;
 template <> struct RawT<2> { using T = unsigned short; };
 template <> struct RawT<4> { using T = unsigned int; };
@@ -75,18 +60,53 @@ __device__ __forceinline__ void load_slice(const S* p, int nv, S (&out)[V]) {
   }
 }
 
-// One whole 16-byte slice at B + row * ldb (row, ldb < 2^32: a single wide
-// 32 x 32-bit multiply), no partial-slice test: the team kernels point lanes
-// without columns at a valid slice and discard what they load.  (L2
-// evict-last hints on these gathers, with evict-first on A and C, measured no
-// better: fp32 N = 128 on a 1,000,000-row power-law matrix kept its 11 % L2
-// hit rate.)
-template <typename S, int V>
-__device__ __forceinline__ void load_row16(const S* __restrict__ B, uint32_t row, uint32_t ldb, S (&out)[V]) {
-  static_assert(int(sizeof(S)) * V == 16, "one 16-byte slice");
-  const uint4 r = __ldg(reinterpret_cast<const uint4*>(B + static_cast<uint64_t>(row) * ldb));
-  memcpy(out, &r, 16);
-}
+// A lane's share of a team's column tile: P pieces of E consecutive elements,
+// a team's T lanes side by side in each piece, piece q of lane tl starting at
+// tile column (q * T + tl) * E.  Aligned rows take one 16-byte piece (P = 1).
+// Other widths take pieces of one element or, where N, the leading dimensions
+// and the addresses allow, of 4 or 8 bytes; each piece lies wholly inside or
+// outside the N columns.
+template <typename S, int E, int P>
+struct Slice {
+  static constexpr int V = E * P;
+  static constexpr bool kWhole = P == 1 && E * int(sizeof(S)) == 16;
+  using Raw = typename RawT<E * int(sizeof(S))>::T;
+  int off[P];  // this lane's first column of each piece, any valid column for pieces past N
+  int nv;      // valid pieces
+
+  __device__ __forceinline__ void set(int64_t tile, int T, int tl, int64_t n) {
+    nv = 0;
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      const int64_t c = (tile * (int64_t(T) * P) + q * T + tl) * E;
+      const bool ok = c < n;
+      off[q] = ok ? static_cast<int>(c) : 0;
+      nv += ok ? 1 : 0;
+    }
+  }
+  // first column's address: whole slices carry their offset in it
+  __device__ __forceinline__ const S* base(const S* B) const { return kWhole ? B + off[0] : B; }
+  // slice of row `row` (whole slices: ldb < 2^32, a single wide 32 x 32-bit multiply)
+  __device__ __forceinline__ void load(const S* __restrict__ base, uint32_t row, int64_t ldb, S (&out)[V]) const {
+    const S* r = base + (kWhole ? static_cast<uint64_t>(row) * static_cast<uint32_t>(ldb)
+                                : static_cast<uint64_t>(row) * static_cast<uint64_t>(ldb));
+#pragma unroll
+    for (int q = 0; q < P; ++q) {
+      const Raw w = __ldg(reinterpret_cast<const Raw*>(r + (kWhole ? 0 : off[q])));
+      memcpy(&out[q * E], &w, sizeof(Raw));
+    }
+  }
+  // streaming (evict-first) stores: the output is written once
+  __device__ __forceinline__ void store(S* __restrict__ row, const S (&v)[V]) const {
+#pragma unroll
+    for (int q = 0; q < P; ++q)
+      if (q < nv) {
+        Raw w;
+        memcpy(&w, &v[q * E], sizeof(Raw));
+        __stcs(reinterpret_cast<Raw*>(row + off[q]), w);
+      }
+  }
+};
 
 // Output slices are written once: STREAM makes them streaming (evict-first)
 // stores, so the output does not displace gathered rows in L2.
@@ -223,13 +243,6 @@ struct SpmmAcc {
   }
 };
 
-// Per-warp shared-memory slice: staged values, columns, the unit's row
-// offsets and each staged nonzero's local row; a multiple of 16 bytes.
-template <typename S>
-constexpr int spmm_warp_smem_bytes() {
-  return (kSpmmBatch * int(sizeof(S)) + kSpmmBatch * 4 + (kSpmmMaxCap + 1) * 4 + kSpmmBatch + 15) & ~15;
-}
-
 template <int DT>
 struct SpmmMinBlocks { static constexpr int value = (DT == FSB_C128) ? 2 : (DT == FSB_F64 || DT == FSB_C64) ? 3 : 4; };
 
@@ -356,170 +369,13 @@ constexpr int64_t kCompensateAbove = 1024;
 template <int DT, bool COMP>
 constexpr bool kCompLong = !COMP && (DT == FSB_F16 || DT == FSB_BF16 || DT == FSB_F32);
 
-// grid: x = groups of kSpmmWarps units, y = column tiles of 32*V columns.
-// pstride: scratch elements per slot; cps: tickets per slot.
-template <int DT, int V, bool COMP>
-__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmMinBlocks<DT>::value)
-k_spmm_csr(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
-           const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
-           typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int64_t pstride, int64_t cps) {
-  using S = typename VT<DT>::Store;
-  using R = typename VT<DT>::Real;
-  using Acc = SpmmAcc<DT, COMP, V>;
-  constexpr int kER = Acc::kNC * 2;  // scratch reals per element
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t unit = int64_t(blockIdx.x) * kSpmmWarps + warp;
-  if (unit >= plan.n_units) return;  // whole warp leaves together
-  const int tile = blockIdx.y;
-  const int64_t c0 = int64_t(tile) * (kSpmmTileLanes * V) + int64_t(lane) * V;  // this lane's first column
-  const int nv = static_cast<int>(n - c0 >= V ? int64_t(V) : (n > c0 ? n - c0 : int64_t(0)));
-
-  unsigned char* wbase = smem_raw + warp * spmm_warp_smem_bytes<S>();
-  S* sh_a = reinterpret_cast<S*>(wbase);
-  int32_t* sh_c = reinterpret_cast<int32_t*>(wbase + kSpmmBatch * sizeof(S));
-  int32_t* sh_off = sh_c + kSpmmBatch;
-  uint8_t* sh_rid = reinterpret_cast<uint8_t*>(sh_off + kSpmmMaxCap + 1);
-
-  const fsb_spmv_unit* ud = plan.units + unit;
-  const int64_t s0 = __ldg(&ud->nnz_begin), s1 = __ldg(&ud->nnz_end);
-  const int32_t row = __ldg(&ud->row), tag = __ldg(&ud->tag);
-
-  auto flush = [&](const Acc& acc, int64_t r) {
-    if (nv > 0) {
-      S o[V];
-      acc.result(o);
-      store_slice(C + r * ldc + c0, nv, o);
-    }
-  };
-
-  if (tag >= 0) {
-    // ------------------------------------------------------------ row block
-    const int nr = tag - row;
-    const int cnt = static_cast<int>(s1 - s0);
-    for (int i = lane; i <= nr; i += 32) sh_off[i] = static_cast<int32_t>(__ldg(ptr + row + i) - s0);
-    for (int k = lane; k < cnt; k += 32) {
-      sh_a[k] = ld_once(data + s0 + k);
-      sh_c[k] = ld_once(col + s0 + k);
-    }
-    __syncwarp();
-    for (int k = lane; k < cnt; k += 32) {  // local row of nonzero k: first i with off[i+1] > k
-      int lo = 0, hi = nr - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (sh_off[mid + 1] > k) hi = mid; else lo = mid + 1;
-      }
-      sh_rid[k] = static_cast<uint8_t>(lo);
-    }
-    for (int i0 = 0; i0 < nr; i0 += 32) {  // empty rows get zero slices
-      const int i = i0 + lane;
-      unsigned m = __ballot_sync(0xffffffffu, i < nr && sh_off[i] == sh_off[i + 1]);
-      while (m) {
-        const int b = __ffs(m) - 1;
-        m &= m - 1;
-        Acc z;
-        z.zero();
-        flush(z, int64_t(row) + i0 + b);
-      }
-    }
-    __syncwarp();
-    if (cnt == 0) return;
-    Acc acc;
-    acc.zero();
-    int cur = sh_rid[0];
-    for (int k = 0; k < cnt; k += kSpmmAhead) {
-      S bv[kSpmmAhead][V];
-#pragma unroll
-      for (int u = 0; u < kSpmmAhead; ++u) {
-        const int kk = k + u < cnt ? k + u : k;
-        load_slice<S, V>(B + int64_t(sh_c[kk]) * ldb + c0, k + u < cnt ? nv : 0, bv[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < kSpmmAhead; ++u) {
-        if (k + u < cnt) {
-          const int r = sh_rid[k + u];
-          if (r != cur) {  // uniform across the warp
-            flush(acc, int64_t(row) + cur);
-            acc.zero();
-            cur = r;
-          }
-          acc.add(sh_a[k + u], bv[u]);
-        }
-      }
-    }
-    flush(acc, int64_t(row) + cur);
-    return;
-  }
-
-  // ------------------------------------------------------------ long-row chunk
-  const int32_t nch = __ldg(&ud->n_chunks), slot = __ldg(&ud->slot);
-  // A2: the accumulator of this row's chunks (Dot2 for long rows, see kCompLong)
-  auto run_chunk = [&](auto proto) {
-    using A2 = decltype(proto);
-    A2 acc;
-    acc.zero();
-    for (int64_t b0 = s0; b0 < s1; b0 += kSpmmBatch) {
-      const int cnt = static_cast<int>(s1 - b0 < kSpmmBatch ? s1 - b0 : int64_t(kSpmmBatch));
-      __syncwarp();
-      for (int k = lane; k < cnt; k += 32) {
-        sh_a[k] = ld_once(data + b0 + k);
-        sh_c[k] = ld_once(col + b0 + k);
-      }
-      __syncwarp();
-      for (int k = 0; k < cnt; k += kSpmmAhead) {
-        S bv[kSpmmAhead][V];
-#pragma unroll
-        for (int u = 0; u < kSpmmAhead; ++u) {
-          const int kk = k + u < cnt ? k + u : k;
-          load_slice<S, V>(B + int64_t(sh_c[kk]) * ldb + c0, k + u < cnt ? nv : 0, bv[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < kSpmmAhead; ++u)
-          if (k + u < cnt) acc.add(sh_a[k + u], bv[u]);
-      }
-    }
-    auto put = [&](const A2& a) {
-      if (nv > 0) {
-        S o[V];
-        a.result(o);
-        store_slice(C + int64_t(row) * ldc + c0, nv, o);
-      }
-    };
-    if (nch == 1) {
-      put(acc);
-      return;
-    }
-    R* part = static_cast<R*>(plan.partials);
-    const int64_t first = int64_t(slot) + (tag + 1);  // slot of the row's first chunk
-    acc.store_partial(part + (int64_t(slot) * pstride + c0) * kER);
-    __threadfence();
-    __syncwarp();
-    int ticket = 0;
-    if (lane == 0) ticket = atomicAdd(plan.counters + first * cps + tile, 1);
-    ticket = __shfl_sync(0xffffffffu, ticket, 0);
-    if (ticket != nch - 1) return;
-    __threadfence();
-    A2 fin;
-    fin.zero();
-#pragma unroll 4
-    for (int c = 0; c < nch; ++c) fin.add_partial(part + ((first + c) * pstride + c0) * kER);
-    put(fin);
-    if (lane == 0) plan.counters[first * cps + tile] = 0;  // ready for the next call
-  };
-  if (kCompLong<DT, COMP> && int64_t(nch) * plan.chunk_nnz > kCompensateAbove)
-    run_chunk(SpmmAcc<DT, true, V>());
-  else
-    run_chunk(Acc());
-}
-
 // ---------------------------------------------------------------------------
-// Dense rows made of whole aligned 16-byte slices: the team kernel.  Teams of
-// T lanes (1 to 32) own the 16-byte slices of a column tile of T * 16 bytes,
-// G = 32 / T teams per warp.  Rows wider than the tile run as several column
-// tiles; the tile is the slowest work dimension, so while one tile is in
-// flight only that tile's slice of B is being gathered, and a slice that fits
-// in L2 is read from HBM about once.
+// The team kernel.  Teams of T lanes (1 to 32) own a column tile, G = 32 / T
+// teams per warp: T * 16 bytes of aligned rows, T * P pieces of others (Slice).
+// Rows wider than the tile run as several column tiles; the tile is the
+// slowest work dimension, so while one tile is in flight only that tile's
+// slice of B is being gathered, and a slice that fits in L2 is read from HBM
+// about once.
 //
 // Persistent warps stride over the work items of every tile in tile order.
 // An item is either
@@ -552,10 +408,9 @@ template <typename S>
 constexpr int spmm_team_park_offset() {
   return (spmm_team_vals_bytes<S>() + kRowStage * 4 + (kRowRows + 1) * 4 + 15) & ~15;
 }
-template <int DT, bool COMP>
+template <int DT, bool COMP, int V>
 constexpr int spmm_team_warp_smem_bytes() {
   using S = typename VT<DT>::Store;
-  constexpr int V = 16 / int(sizeof(S));
   return spmm_team_park_offset<S>() + 32 * int(sizeof(SpmmAcc<DT, COMP, V>));
 }
 
@@ -564,9 +419,12 @@ constexpr int spmm_team_warp_smem_bytes() {
 // compensated or fused sums, 2 for complex fp64.  More resident warps keep
 // more B rows in flight: wide rows measured up to 15 % faster at 4 blocks with
 // 4 slices ahead than at 3 blocks with 6 ahead.
-template <int DT, bool COMP, bool FUSED, int KP>
+// Three or four pieces per lane spill at 64 registers: 80 against 87 us at 3
+// blocks (47 columns of fp32, a 170,001-row Chung-Lu graph).
+template <int DT, bool COMP, bool FUSED, int P>
 struct SpmmTeamMinBlocks {
-  static constexpr int value = (DT == FSB_C128) ? 2 : (!COMP && !FUSED && DT != FSB_F64 && DT != FSB_C64) ? 4 : 3;
+  static constexpr int value =
+      (DT == FSB_C128) ? 2 : (!COMP && !FUSED && P < 3 && DT != FSB_F64 && DT != FSB_C64) ? 4 : 3;
 };
 
 // B-row slices a team loads ahead of its sums in the row walk (KP): 4 for
@@ -692,27 +550,29 @@ struct ChunkAcc<DT, 3, V> { using T = WideAcc<DT, V>; };
 // KA B-row slices in flight; the team partials are combined by xor-shuffles
 // over the team index, then the chunk is stored directly (one-chunk rows) or
 // as a slot partial whose ticket's last taker adds the partials in chunk order.
-template <int DT, int MODE, bool FUSED, int KA>
+template <int DT, int MODE, bool FUSED, int KA, int E, int P>
 __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restrict__ data,
                                            const int32_t* __restrict__ col,
-                                           const typename VT<DT>::Store* __restrict__ B, uint32_t ldb, int64_t n,
+                                           const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
                                            typename VT<DT>::Store* __restrict__ C, int64_t ldc,
                                            const fsb_spmv_plan& plan, const fsb_spmv_unit* ud, int T, int64_t tile,
-                                           int64_t c0, int nv, int64_t pstride, int64_t cps,
+                                           const Slice<typename VT<DT>::Store, E, P>& sl, int64_t pstride,
+                                           int64_t cps,
                                            const typename VT<DT>::Store* __restrict__ x,
                                            typename VT<DT>::Store* __restrict__ y, typename VT<DT>::Store* sh_a,
                                            int32_t* sh_c) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
-  constexpr int V = 16 / int(sizeof(S));
+  constexpr int V = E * P;
   using Acc = typename ChunkAcc<DT, MODE, V>::T;
   constexpr int kER = Acc::kNC * 2;
   const int lane = threadIdx.x & 31;
   const int G = 32 / T, team = lane / T;
+  const int64_t c0 = (tile * T + lane % T) * V;  // this lane's place in a slot's partials
   const int64_t s0 = __ldg(&ud->nnz_begin), s1 = __ldg(&ud->nnz_end);
   const int32_t row = __ldg(&ud->row), tag = __ldg(&ud->tag);
   const int32_t nch = __ldg(&ud->n_chunks), slot = __ldg(&ud->slot);
-  const S* Bl = B + (nv > 0 ? c0 : 0);  // lanes without columns load column 0 and discard it
+  const S* Bl = sl.base(B);
   Acc acc;
   acc.zero();
   YAcc<R> yacc;
@@ -728,7 +588,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
 #pragma unroll
       for (int q = 0; q < KA; ++q) {
         const int kk = k + q * G + team;
-        load_row16<S, V>(Bl, static_cast<uint32_t>(sh_c[kk < cnt ? kk : cnt - 1]), ldb, bv[q]);
+        sl.load(Bl, static_cast<uint32_t>(sh_c[kk < cnt ? kk : cnt - 1]), ldb, bv[q]);
       }
       if constexpr (FUSED) {
         // the y terms of these KA * G items, one per lane in order
@@ -769,10 +629,10 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
     for (int m = 1; m < 32; m <<= 1) yacc.shfl_join(m);
   }
   if (nch == 1) {
-    if (team == 0 && nv > 0) {
+    if (team == 0 && sl.nv > 0) {
       S o[V];
       acc.result(o);
-      store_slice<S, V, true>(C + int64_t(row) * ldc + c0, nv, o);
+      sl.store(C + int64_t(row) * ldc, o);
     }
     if constexpr (FUSED)
       if (lane == 0 && tile == 0) put_y(y[row], yacc.value());
@@ -797,10 +657,10 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
     fin.zero();
 #pragma unroll 4
     for (int c = 0; c < nch; ++c) fin.add_partial(part + ((first + c) * pstride + c0) * kER);
-    if (nv > 0) {
+    if (sl.nv > 0) {
       S o[V];
       fin.result(o);
-      store_slice<S, V, true>(C + int64_t(row) * ldc + c0, nv, o);
+      sl.store(C + int64_t(row) * ldc, o);
     }
     if constexpr (FUSED) {
       if (lane == 0 && tile == 0) {
@@ -814,16 +674,16 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
   }
 }
 
-template <int DT, bool COMP, bool FUSED, int KP>
-__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmTeamMinBlocks<DT, COMP, FUSED, KP>::value)
+template <int DT, bool COMP, bool FUSED, int KP, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
+__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmTeamMinBlocks<DT, COMP, FUSED, P>::value)
 k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
-            const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, uint32_t ldb, int64_t n,
+            const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
             typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int T, int64_t tiles,
             int64_t pstride, int64_t cps, const typename VT<DT>::Store* __restrict__ x,
             typename VT<DT>::Store* __restrict__ y) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
-  constexpr int V = 16 / int(sizeof(S));
+  constexpr int V = E * P;
   using Acc = SpmmAcc<DT, COMP, V>;
   constexpr int kP = KP;
   // the KP != 4 instantiation runs 32-lane teams only (one team per warp): a
@@ -833,7 +693,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int G = 32 / T, team = lane / T, tl = lane % T;
-  unsigned char* wbase = smem_raw + warp * spmm_team_warp_smem_bytes<DT, COMP>();
+  unsigned char* wbase = smem_raw + warp * spmm_team_warp_smem_bytes<DT, COMP, V>();
   S* sh_a = reinterpret_cast<S*>(wbase);
   int32_t* sh_c = reinterpret_cast<int32_t*>(wbase + spmm_team_vals_bytes<S>());
   int32_t* sh_off = sh_c + kRowStage;
@@ -847,9 +707,9 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
 
   for (uint32_t it = blockIdx.x * kSpmmWarps + warp; it < total; it += nwarps) {
     const uint32_t tile = it / n_items, item = it - tile * n_items;
-    const int64_t c0 = int64_t(tile) * (int64_t(T) * V) + int64_t(tl) * V;  // this lane's first column
-    const int nv = c0 + V <= n ? V : 0;                       // n is a multiple of V
-    const S* Bl = B + (nv > 0 ? c0 : 0);  // lanes without columns load column 0 and discard it
+    Slice<S, E, P> sl;  // pieces past N load column 0 and are not stored
+    sl.set(tile, T, tl, n);
+    const S* Bl = sl.base(B);
     __syncwarp();  // the staging slice of the previous item is free
 
     if (item < n_groups) {
@@ -897,12 +757,12 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
             const int b = __ffs(m) - 1;
             m &= m - 1;
             if (q % G == team) {
-              if (nv > 0) {
+              if (sl.nv > 0) {
                 Acc z;
                 z.zero();
                 S o[V];
                 z.result(o);
-                store_slice<S, V, true>(C + (int64_t(r0) + i0 + b) * ldc + c0, nv, o);
+                sl.store(C + (int64_t(r0) + i0 + b) * ldc, o);
               }
               if constexpr (FUSED)
                 if (tl == 0 && tile == 0) put_y(y[int64_t(r0) + i0 + b], 0.0f);
@@ -935,10 +795,10 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
         bool open_start = jb < je && sh_off[cur] < jb;  // row cur began in an earlier team
         int park_row = -1;
         auto put_row = [&](const Acc& a, const YAcc<R>& ya, int r) {
-          if (nv > 0) {
+          if (sl.nv > 0) {
             S o[V];
             a.result(o);
-            store_slice<S, V, true>(C + (int64_t(r0) + r) * ldc + c0, nv, o);
+            sl.store(C + (int64_t(r0) + r) * ldc, o);
           }
           if constexpr (FUSED)
             if (tl == 0 && tile == 0) put_y(y[int64_t(r0) + r], ya.value());
@@ -949,7 +809,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
 #pragma unroll
           for (int q = 0; q < kP; ++q) {  // past je: the last nonzero again, loaded and not summed
             const int j = j0 + q < je ? j0 + q : je - 1;
-            load_row16<S, V>(Bl, static_cast<uint32_t>(sh_c[j]), ldb, bv[q]);
+            sl.load(Bl, static_cast<uint32_t>(sh_c[j]), ldb, bv[q]);
             if constexpr (FUSED) xv[q] = ld_gather(x + sh_c[j]);
           }
 #pragma unroll
@@ -1033,19 +893,19 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     // fp32-accumulated types, partials and all (blocked Dot2, or fp64 sums
     // in the one-team kernel)
     if constexpr (COMP) {
-      team_chunk<DT, 1, FUSED, KP>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, c0, nv, pstride, cps, x, y,
-                                   sh_a, sh_c);
+      team_chunk<DT, 1, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl, pstride, cps, x, y, sh_a,
+                                         sh_c);
       continue;
     }
     if constexpr (kCompLong<DT, COMP>) {
       if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
-        team_chunk<DT, (KP > kSpmmAhead ? 3 : 2), FUSED, KP>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, c0, nv,
-                                                             pstride, cps, x, y, sh_a, sh_c);
+        team_chunk<DT, (KP > kSpmmAhead ? 3 : 2), FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
+                                                                   pstride, cps, x, y, sh_a, sh_c);
         continue;
       }
     }
-    team_chunk<DT, 0, FUSED, KP>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, c0, nv, pstride, cps, x, y, sh_a,
-                                 sh_c);
+    team_chunk<DT, 0, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl, pstride, cps, x, y, sh_a,
+                                       sh_c);
   }
 }
 
@@ -1399,51 +1259,21 @@ inline int spmm_team_tile_bytes(int64_t row_bytes, int32_t hint) {
   return w;
 }
 
-template <int DT, int V, bool COMP>
-int spmm_launch_v(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
-                  void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
-  using S = typename VT<DT>::Store;
-  const int64_t tiles = ceil_div(n, kSpmmTileLanes * V);
-  if (tiles > 65535) return FSB_ERR_UNSUPPORTED;
-  const int64_t blocks = ceil_div(plan.n_units, kSpmmWarps);
-  const size_t smem = size_t(spmm_warp_smem_bytes<S>()) * kSpmmWarps;
-  dim3 grid((unsigned)blocks, (unsigned)tiles);
-  k_spmm_csr<DT, V, COMP><<<grid, kSpmmWarps * 32, smem, st>>>(
-      static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), ldb, n, static_cast<S*>(C), ldc, plan,
-      spmm_pstride(n), spmm_cps<DT>(n));
-  FSB_LAUNCH_CHECK();
-  return FSB_OK;
-}
-
-// Widest per-lane vector (elements) that 32 lanes need for N columns and that
-// the B / C base addresses and leading dimensions allow.
-template <int DT>
-int spmm_pick_v(const void* B, int64_t ldb, const void* C, int64_t ldc, int64_t n) {
-  using S = typename VT<DT>::Store;
-  constexpr int kVmax = 16 / int(sizeof(S));
-  int v = 1;
-  while (v < kVmax && int64_t(kSpmmTileLanes) * v < n) v *= 2;
-  auto ok = [&](int w) {
-    const uintptr_t a = uintptr_t(w) * sizeof(S);
-    return reinterpret_cast<uintptr_t>(B) % a == 0 && reinterpret_cast<uintptr_t>(C) % a == 0 && ldb % w == 0 &&
-           ldc % w == 0;
-  };
-  while (v > 1 && !ok(v)) v /= 2;
-  return v;
-}
-
 // The team kernel: one work item per warp, the items of every tile in tile
 // order (tile bytes = T * 16), so the blocks of one tile run together; with
 // FSB_SPMM_PERSISTENT, the resident blocks, whose warps stride over the items
 // in the same order.
-template <int DT, bool COMP, bool FUSED = false>
+template <int DT, bool COMP, bool FUSED = false, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
 int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
                      void* C, int64_t ldc, const fsb_spmv_plan& plan, int T, int64_t tiles, cudaStream_t st,
                      const void* x = nullptr, void* y = nullptr) {
   using S = typename VT<DT>::Store;
-  const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP>()) * kSpmmWarps;
-  const int wide = (!FUSED && T == 32) ? 1 : 0;
-  auto kern = wide ? k_spmm_team<DT, COMP, FUSED, 6> : k_spmm_team<DT, COMP, FUSED, 4>;
+  constexpr bool kAligned = P == 1 && E * int(sizeof(S)) == 16;
+  const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kSpmmWarps;
+  const int wide = (kAligned && !FUSED && T == 32) ? 1 : 0;
+  auto kern = k_spmm_team<DT, COMP, FUSED, 4, E, P>;
+  if constexpr (kAligned)
+    if (wide) kern = k_spmm_team<DT, COMP, FUSED, 6, E, P>;
   if (smem > 48 * 1024) {  // opt in to the larger dynamic shared memory once per kernel and device
     static std::atomic<uint64_t> done[2];
     int dev = 0;
@@ -1463,7 +1293,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
   const int64_t nb = plan.n_block_units;
   const int64_t items = (ceil_div(nb, kRowUnits) + (plan.n_units - nb)) * tiles;
   int64_t blocks = ceil_div(items, kSpmmWarps);  // one work item per warp, tiles in block order
-  if (items >= (int64_t(1) << 32) || blocks > INT32_MAX || ldb > UINT32_MAX) return FSB_ERR_UNSUPPORTED;
+  if (items >= (int64_t(1) << 32) || blocks > INT32_MAX || (kAligned && ldb > UINT32_MAX)) return FSB_ERR_UNSUPPORTED;
   if (blocks < 1) return FSB_OK;
   if (plan.flags & FSB_SPMM_PERSISTENT) {  // the resident blocks; warps stride over the items
     static std::atomic<int64_t> resident[2][64];
@@ -1487,7 +1317,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
     if (blocks > r) blocks = r;
   }
   kern<<<(unsigned)blocks, kSpmmWarps * 32, smem, st>>>(
-      static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), static_cast<uint32_t>(ldb), n,
+      static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), ldb, n,
       static_cast<S*>(C), ldc, plan, T, tiles, spmm_pstride(n), spmm_cps<DT>(n), static_cast<const S*>(x),
       static_cast<S*>(y));
   FSB_LAUNCH_CHECK();
@@ -1554,6 +1384,34 @@ int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, con
   }
 }
 
+// Rows of E-element pieces (see Slice): teams of T lanes with P pieces of at
+// most 16 bytes together, as few lanes as hold a tile's pieces, so that a warp
+// runs as many teams as it can; at most 32 * kMaxP pieces per column tile,
+// spread evenly over the tiles.  One warp per unit and 32-column tile, which
+// this replaced, left most lanes idle on narrow rows and ran two passes at 33
+// to 64 columns (fp32 on a 170,001-row Chung-Lu graph, 47 columns: 208 -> 89
+// us; 300,000 rows, 5 columns: 219 -> 84 us; 129 columns: 1543 -> 872 us).
+template <int DT, bool COMP, int E>
+int spmm_launch_pieces(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
+                       void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
+  constexpr int kFit = 16 / (E * int(sizeof(typename VT<DT>::Store)));
+  constexpr int kMaxP = kFit < 4 ? kFit : 4;
+  const int64_t pieces = n / E;
+  const int per = static_cast<int>(ceil_div(pieces, ceil_div(pieces, 32 * kMaxP)));
+  int T = 1;
+  while (T * kMaxP < per) T *= 2;
+  const int P = (per + T - 1) / T;
+  const int64_t tiles = ceil_div(pieces, int64_t(T) * P);
+  if (n > INT32_MAX || tiles * T * P * E > spmm_pstride(n)) return FSB_ERR_UNSUPPORTED;
+  if constexpr (kMaxP >= 4) {
+    if (P == 4) return spmm_launch_team<DT, COMP, false, E, 4>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, tiles, st);
+    if (P == 3) return spmm_launch_team<DT, COMP, false, E, 3>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, tiles, st);
+  }
+  if constexpr (kMaxP >= 2)
+    if (P == 2) return spmm_launch_team<DT, COMP, false, E, 2>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, tiles, st);
+  return spmm_launch_team<DT, COMP, false, E, 1>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, tiles, st);
+}
+
 template <int DT, bool COMP>
 int spmm_dispatch(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
                   int64_t n_cols, void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
@@ -1562,20 +1420,27 @@ int spmm_dispatch(const void* data, const int32_t* idx, const int64_t* ptr, cons
   // rows of whole, aligned 16-byte slices: teams of T lanes over column tiles
   // of T * 16 bytes (spmm_team_tile_bytes)
   if (n % kVmax == 0 && ldb % kVmax == 0 && ldc % kVmax == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldb <= UINT32_MAX && n_cols < (int64_t(1) << 32)) {
+      reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldb <= UINT32_MAX && n <= INT32_MAX) {
     const int w = spmm_team_tile_bytes(n * int64_t(sizeof(S)), plan.tile_bytes);
     const int T = w / 16;
     return spmm_launch_team<DT, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, ceil_div(n, int64_t(T) * kVmax),
                                       st);
   }
-  const int v = spmm_pick_v<DT>(B, ldb, C, ldc, n);
-  if constexpr (kVmax >= 8)
-    if (v == 8) return spmm_launch_v<DT, 8, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
-  if constexpr (kVmax >= 4)
-    if (v == 4) return spmm_launch_v<DT, 4, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
-  if constexpr (kVmax >= 2)
-    if (v == 2) return spmm_launch_v<DT, 2, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
-  return spmm_launch_v<DT, 1, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
+  // other widths and addresses: pieces of 8 or 4 bytes where everything is a
+  // multiple of them, else of one element
+  auto fits = [&](int e) {
+    const uintptr_t a = uintptr_t(e) * sizeof(S);
+    return n % e == 0 && ldb % e == 0 && ldc % e == 0 && reinterpret_cast<uintptr_t>(B) % a == 0 &&
+           reinterpret_cast<uintptr_t>(C) % a == 0;
+  };
+  if constexpr (sizeof(S) == 2) {
+    if (fits(4)) return spmm_launch_pieces<DT, COMP, 4>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
+    if (fits(2)) return spmm_launch_pieces<DT, COMP, 2>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
+  } else if constexpr (sizeof(S) == 4) {
+    if (fits(2)) return spmm_launch_pieces<DT, COMP, 2>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
+  }
+  if constexpr (sizeof(S) == 16) return FSB_ERR_UNSUPPORTED;  // an element is a slice: B or C is misaligned
+  else return spmm_launch_pieces<DT, COMP, 1>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
 }
 
 template <int DT>

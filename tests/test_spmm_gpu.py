@@ -321,6 +321,33 @@ def test_spmm_persistent_grid_bitwise(dname, N, tile):
     assert torch.equal(C[0], C[1]) and torch.equal(ys[0], ys[1])
 
 
+@pytest.mark.parametrize("dname", ["float32", "bfloat16", "float64", "complex64"])
+@pytest.mark.parametrize("N", [2, 3, 6, 7, 9, 31, 33, 47, 50, 97, 127, 129, 132, 258])
+@pytest.mark.parametrize("gap", [0, 1])
+def test_spmm_piece_widths(dname, N, gap):
+    """Widths and leading dimensions off the 16-byte slices: every piece size, one to four pieces
+    per lane, several column tiles, rows in one and in many chunks, empty rows; columns past N of
+    a wider C stay untouched."""
+    lens = np.array([0, 1, 3, 0, 0, 17, 64, 65, 300, 5, 2500, 0, 30, 1] + [2] * 70 + [0, 9], dtype=np.int64)
+    ptr = np.concatenate([[0], np.cumsum(lens)])
+    k = 3000
+    rng = np.random.Generator(np.random.PCG64(N))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int64)
+    cplx = dname.startswith("complex")
+    draw = lambda *shape: rng.standard_normal(shape) + (1j * rng.standard_normal(shape) if cplx else 0)
+    data, B = draw(idx.size), draw(k, N)
+    dt = TORCH_DT[dname]
+    plan = _csr.SpmmPlan(dev(ptr), lens.size, dt)
+    Bw = torch.zeros(k, N + gap, dtype=dt, device="cuda")
+    Cw = torch.full((lens.size, N + gap), 7.0, dtype=dt, device="cuda")
+    Bw[:, :N] = dev(B, dt)
+    C = _csr.spmm(dev(data, dt), dev(idx, torch.int32), dev(ptr), lens.size, k, Bw[:, :N], plan, Cw[:, :N])
+    assert plan.n_slots > 0 and plan.counters_clear()
+    assert gap == 0 or bool((Cw[:, N:] == 7.0).all())
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(data, dname), (lens.size, k), rounded(B, dname), "non")
+    _check(C.contiguous(), ref, scale, n, dname, f"{dname} N={N} gap={gap}")
+
+
 # ---------------------------------------------------------------- opt entry points / API contract
 
 def test_spmm_opt_entry_points_agree():
