@@ -29,7 +29,15 @@
 namespace fsb {
 namespace {
 
-constexpr int kSpmmWarps = 8;      // warps per block; one (unit, tile) per warp
+// Warps per block, one work item (or unit) per warp.  Items are uneven, and a
+// block's place is free only when its last warp ends: blocks of 2 warps instead
+// of 8 keep more warps resident (1 M-row power-law matrix, 128 columns: bf16
+// 1.54 -> 1.30 ms, fp32 2.35 -> 2.16 ms; single warps: 1.25 / 2.90 ms).  The
+// fused kernel of the batched step stays at 8: its persistent grid levels the
+// items itself (256 uneven matrices: 1.90 against 2.02 ms).
+constexpr int kSpmmWarps = 2;
+template <bool FUSED>
+constexpr int kTeamWarps = FUSED ? 8 : kSpmmWarps;
 constexpr int kSpmmBatch = 128;    // nonzeros staged per batch
 constexpr int kSpmmMaxCap = 64;    // row blocks hold < 2*cap <= kSpmmBatch nonzeros
 constexpr int kSpmmAhead = 4;      // B slices loaded ahead of the multiply-adds
@@ -243,8 +251,9 @@ struct SpmmAcc {
   }
 };
 
+// resident warps of the backward, in units of 8
 template <int DT>
-struct SpmmMinBlocks { static constexpr int value = (DT == FSB_C128) ? 2 : (DT == FSB_F64 || DT == FSB_C64) ? 3 : 4; };
+struct SpmmBwdWarps8 { static constexpr int value = (DT == FSB_C128) ? 2 : (DT == FSB_F64 || DT == FSB_C64) ? 3 : 4; };
 
 // Gather of x for the fused y sums: L2-only.
 template <typename T> __device__ __forceinline__ T ld_gather(const T* p) { return __ldcg(p); }
@@ -414,15 +423,15 @@ constexpr int spmm_team_warp_smem_bytes() {
   return spmm_team_park_offset<S>() + 32 * int(sizeof(SpmmAcc<DT, COMP, V>));
 }
 
-// Resident blocks the register budget is sized for: 4 (64 registers) for
-// plain sums of 2- and 4-byte values, 3 (85) for 8-byte values and for
-// compensated or fused sums, 2 for complex fp64.  More resident warps keep
-// more B rows in flight: wide rows measured up to 15 % faster at 4 blocks with
-// 4 slices ahead than at 3 blocks with 6 ahead.
-// Three or four pieces per lane spill at 64 registers: 80 against 87 us at 3
-// blocks (47 columns of fp32, a 170,001-row Chung-Lu graph).
+// Resident warps the register budget is sized for, in units of 8: 4 (64
+// registers) for plain sums of 2- and 4-byte values, 3 (85) for 8-byte values
+// and for compensated or fused sums, 2 for complex fp64.  More resident warps
+// keep more B rows in flight: wide rows measured up to 15 % faster at 4 units
+// with 4 slices ahead than at 3 with 6 ahead.  Three or four pieces per lane
+// spill at 64 registers: 80 against 87 us at 3 units (47 columns of fp32, a
+// 170,001-row Chung-Lu graph).
 template <int DT, bool COMP, bool FUSED, int P>
-struct SpmmTeamMinBlocks {
+struct SpmmTeamWarps8 {
   static constexpr int value =
       (DT == FSB_C128) ? 2 : (!COMP && !FUSED && P < 3 && DT != FSB_F64 && DT != FSB_C64) ? 4 : 3;
 };
@@ -546,6 +555,45 @@ struct ChunkAcc<DT, 2, V> { using T = SpmmAcc<DT, true, V>; };
 template <int DT, int V>
 struct ChunkAcc<DT, 3, V> { using T = WideAcc<DT, V>; };
 
+// How a long row's chunk partials are joined, in fixed order.  Up to
+// kJoinChunks chunks: the warp that takes the row's last ticket adds them all.
+// More: the last of each group of kJoinChunks adds its group's partials into
+// the group's first slot, and the last group adds the groups', so the longest
+// rows (50,000 nonzeros: 196 chunks) end after two short sums instead of one
+// warp's long one.  A row's ticket counts at its first slot, a group's at the
+// group's second slot (a group of one takes none).
+constexpr int kJoinChunks = 16;
+struct ChunkJoin {
+  int64_t group_slot;  // first slot of the chunk's group
+  int group_size;      // chunks in it
+  int members;         // partials of the row's final sum
+  int64_t step;        // their distance in slots
+  __device__ __forceinline__ ChunkJoin(int nch, int chunk, int64_t first) {
+    const int g = chunk / kJoinChunks;
+    const bool split = nch > kJoinChunks;
+    group_slot = first + int64_t(g) * kJoinChunks;
+    group_size = split ? min(kJoinChunks, nch - g * kJoinChunks) : 1;
+    members = split ? (nch + kJoinChunks - 1) / kJoinChunks : nch;
+    step = split ? kJoinChunks : 1;
+  }
+  __device__ __forceinline__ bool grouped() const { return group_size > 1; }
+  __device__ __forceinline__ int64_t group_ticket() const { return group_slot + 1; }
+};
+
+// The warp's partial is stored: take a ticket; true for the last of `count`,
+// after which every partial can be read and the ticket is zero again.
+__device__ __forceinline__ bool join_ticket(int32_t* counter, int count, int lane) {
+  __threadfence();
+  __syncwarp();
+  int ticket = 0;
+  if (lane == 0) ticket = atomicAdd(counter, 1);
+  ticket = __shfl_sync(0xffffffffu, ticket, 0);
+  if (ticket != count - 1) return false;
+  __threadfence();
+  if (lane == 0) *counter = 0;  // ready for the next call
+  return true;
+}
+
 // One long-row chunk of the team kernel: team g takes nonzeros g, g+G, ...,
 // KA B-row slices in flight; the team partials are combined by xor-shuffles
 // over the team index, then the chunk is stored directly (one-chunk rows) or
@@ -645,37 +693,43 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
     // y's partial sits in the slot's column n (n < pstride for the fused path)
     if (lane == 0 && tile == 0) yacc.store(part + (int64_t(slot) * pstride + n) * kER);
   }
-  __threadfence();
-  __syncwarp();
-  int ticket = 0;
-  if (lane == 0) ticket = atomicAdd(plan.counters + first * cps + tile, 1);
-  ticket = __shfl_sync(0xffffffffu, ticket, 0);
-  if (ticket != nch - 1) return;
-  __threadfence();
-  if (team == 0) {
+  // the sum of partials from, from + step, ... (count of them) in this order,
+  // on every team
+  auto total = [&](int64_t from, int64_t step, int count) {
     Acc fin;
     fin.zero();
 #pragma unroll 4
-    for (int c = 0; c < nch; ++c) fin.add_partial(part + ((first + c) * pstride + c0) * kER);
-    if (sl.nv > 0) {
-      S o[V];
-      fin.result(o);
-      sl.store(C + int64_t(row) * ldc, o);
-    }
-    if constexpr (FUSED) {
-      if (lane == 0 && tile == 0) {
-        YAcc<R> fy;
-        fy.zero();
-        for (int c = 0; c < nch; ++c) fy.add_stored(part + ((first + c) * pstride + n) * kER);
-        put_y(y[row], fy.value());
-      }
-    }
-    if (lane == 0) plan.counters[first * cps + tile] = 0;  // ready for the next call
+    for (int c = team; c < count; c += G) fin.add_partial(part + ((from + c * step) * pstride + c0) * kER);
+    for (int m = T; m < 32; m <<= 1) acc_shfl_add(fin, m);
+    return fin;
+  };
+  auto total_y = [&](int64_t from, int64_t step, int count) {
+    YAcc<R> fy;
+    fy.zero();
+    for (int c = 0; c < count; ++c) fy.add_stored(part + ((from + c * step) * pstride + n) * kER);
+    return fy;
+  };
+  const ChunkJoin join(nch, -(tag + 1), first);
+  if (join.grouped()) {
+    if (!join_ticket(plan.counters + join.group_ticket() * cps + tile, join.group_size, lane)) return;
+    const Acc g = total(join.group_slot, 1, join.group_size);
+    if (team == 0) g.store_partial(part + (join.group_slot * pstride + c0) * kER);
+    if constexpr (FUSED)
+      if (lane == 0 && tile == 0) total_y(join.group_slot, 1, join.group_size).store(part + (join.group_slot * pstride + n) * kER);
   }
+  if (!join_ticket(plan.counters + first * cps + tile, join.members, lane)) return;
+  const Acc fin = total(first, join.step, join.members);
+  if (team == 0 && sl.nv > 0) {
+    S o[V];
+    fin.result(o);
+    sl.store(C + int64_t(row) * ldc, o);
+  }
+  if constexpr (FUSED)
+    if (lane == 0 && tile == 0) put_y(y[row], total_y(first, join.step, join.members).value());
 }
 
 template <int DT, bool COMP, bool FUSED, int KP, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
-__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmTeamMinBlocks<DT, COMP, FUSED, P>::value)
+__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, P>::value * 8 / kTeamWarps<FUSED>)
 k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
             const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
             typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int T, int64_t tiles,
@@ -703,9 +757,9 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
   const uint32_t n_groups = static_cast<uint32_t>(ceil_div(nb, kRowUnits));
   const uint32_t n_items = n_groups + static_cast<uint32_t>(plan.n_units - nb);
   const uint32_t total = n_items * static_cast<uint32_t>(tiles);
-  const uint32_t nwarps = gridDim.x * kSpmmWarps;
+  const uint32_t nwarps = gridDim.x * kTeamWarps<FUSED>;
 
-  for (uint32_t it = blockIdx.x * kSpmmWarps + warp; it < total; it += nwarps) {
+  for (uint32_t it = blockIdx.x * kTeamWarps<FUSED> + warp; it < total; it += nwarps) {
     const uint32_t tile = it / n_items, item = it - tile * n_items;
     Slice<S, E, P> sl;  // pieces past N load column 0 and are not stored
     sl.set(tile, T, tl, n);
@@ -1034,7 +1088,7 @@ __device__ __forceinline__ void bwd_put_dots(R (&d)[KA], int base, int stride, i
 }
 
 template <int DT, bool DV>
-__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmMinBlocks<DT>::value)
+__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmBwdWarps8<DT>::value * 8 / kSpmmWarps)
 k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __restrict__ perm,
            const int32_t* __restrict__ col, const int64_t* __restrict__ ptr,
            const typename VT<DT>::Store* __restrict__ dY, int64_t lddy, int64_t n,
@@ -1180,24 +1234,27 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
     R* part = static_cast<R*>(plan.partials);
     const int64_t first = int64_t(slot) + (tag + 1);
     if (team == 0) acc.store_partial(part + (int64_t(slot) * pstride + c0) * kER);
-    __threadfence();
-    __syncwarp();
-    int ticket = 0;
-    if (lane == 0) ticket = atomicAdd(plan.counters + first * cps, 1);
-    ticket = __shfl_sync(0xffffffffu, ticket, 0);
-    if (ticket != nch - 1) return;
-    __threadfence();
-    if (team != 0) return;
-    A2 fin;
-    fin.zero();
+    auto total = [&](int64_t from, int64_t step, int count) {
+      A2 fin;
+      fin.zero();
 #pragma unroll 4
-    for (int c = 0; c < nch; ++c) fin.add_partial(part + ((first + c) * pstride + c0) * kER);
-    if (nv > 0) {
+      for (int c = team; c < count; c += G) fin.add_partial(part + ((from + c * step) * pstride + c0) * kER);
+      for (int m = T; m < 32; m <<= 1) acc_shfl_add(fin, m);
+      return fin;
+    };
+    const ChunkJoin join(nch, -(tag + 1), first);
+    if (join.grouped()) {
+      if (!join_ticket(plan.counters + join.group_ticket() * cps, join.group_size, lane)) return;
+      const A2 g = total(join.group_slot, 1, join.group_size);
+      if (team == 0) g.store_partial(part + (join.group_slot * pstride + c0) * kER);
+    }
+    if (!join_ticket(plan.counters + first * cps, join.members, lane)) return;
+    const A2 fin = total(first, join.step, join.members);
+    if (team == 0 && nv > 0) {
       S o[V];
       fin.result(o);
       store_slice<S, V, true>(dX + int64_t(row) * lddx + c0, nv, o);
     }
-    if (lane == 0) plan.counters[first * cps] = 0;  // ready for the next call
   };
   if constexpr (kCompLong<DT, false>) {
     if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
@@ -1269,7 +1326,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
                      const void* x = nullptr, void* y = nullptr) {
   using S = typename VT<DT>::Store;
   constexpr bool kAligned = P == 1 && E * int(sizeof(S)) == 16;
-  const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kSpmmWarps;
+  const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kTeamWarps<FUSED>;
   const int wide = (kAligned && !FUSED && T == 32) ? 1 : 0;
   auto kern = k_spmm_team<DT, COMP, FUSED, 4, E, P>;
   if constexpr (kAligned)
@@ -1292,7 +1349,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
   }
   const int64_t nb = plan.n_block_units;
   const int64_t items = (ceil_div(nb, kRowUnits) + (plan.n_units - nb)) * tiles;
-  int64_t blocks = ceil_div(items, kSpmmWarps);  // one work item per warp, tiles in block order
+  int64_t blocks = ceil_div(items, kTeamWarps<FUSED>);  // one work item per warp, tiles in block order
   if (items >= (int64_t(1) << 32) || blocks > INT32_MAX || (kAligned && ldb > UINT32_MAX)) return FSB_ERR_UNSUPPORTED;
   if (blocks < 1) return FSB_OK;
   if (plan.flags & FSB_SPMM_PERSISTENT) {  // the resident blocks; warps stride over the items
@@ -1305,7 +1362,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
     int64_t r = resident[wide][dev].load(std::memory_order_acquire);
     if (r == 0) {
       int per_sm = 0, sms = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSpmmWarps * 32, smem) != cudaSuccess ||
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTeamWarps<FUSED> * 32, smem) != cudaSuccess ||
           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1 ||
           sms < 1) {
         (void)cudaGetLastError();
@@ -1316,7 +1373,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
     }
     if (blocks > r) blocks = r;
   }
-  kern<<<(unsigned)blocks, kSpmmWarps * 32, smem, st>>>(
+  kern<<<(unsigned)blocks, kTeamWarps<FUSED> * 32, smem, st>>>(
       static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), ldb, n,
       static_cast<S*>(C), ldc, plan, T, tiles, spmm_pstride(n), spmm_cps<DT>(n), static_cast<const S*>(x),
       static_cast<S*>(y));

@@ -348,6 +348,42 @@ def test_spmm_piece_widths(dname, N, gap):
     _check(C.contiguous(), ref, scale, n, dname, f"{dname} N={N} gap={gap}")
 
 
+@pytest.mark.parametrize("dname,N", [("float32", 16), ("float32", 47), ("float32", 128), ("bfloat16", 64),
+                                    ("float64", 8)])
+def test_spmm_long_row_joins(dname, N):
+    """Rows of 1 to 200 chunks: one ticket up to 16 chunks, grouped tickets beyond (groups of 16,
+    a last group of one, of two, full).  Products, the fused y and the backward's dX against the
+    oracle, bitwise the same on a second call, tickets left at zero."""
+    lens = np.array([n * 128 + d for n in (1, 2, 15, 16, 17, 18, 32, 33, 48, 49, 200) for d in (0, -1)] + [0, 3])
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    k = 26_000
+    rng = np.random.Generator(np.random.PCG64(N))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int32)
+    dt = TORCH_DT[dname]
+    data, B, x = rng.standard_normal(idx.size), rng.standard_normal((k, N)), rng.standard_normal(k)
+    d, i, pt, Bd, xd = dev(data, dt), dev(idx), dev(ptr), dev(B, dt), dev(x, dt)
+    plan = _csr.SpmmPlan(pt, lens.size, dt, chunk_nnz=128)
+    C = [torch.empty(lens.size, N, dtype=dt, device="cuda") for _ in range(2)]
+    for C_i in C:
+        _csr.spmm(d, i, pt, lens.size, k, Bd, plan, C_i)
+    assert torch.equal(C[0], C[1]) and plan.counters_clear()
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(data, dname), (lens.size, k), rounded(B, dname), "non")
+    _check(C[0], ref, scale, n, dname, f"{dname} N={N}")
+    if N * d.element_size() <= 256 and N % (16 // d.element_size()) == 0:
+        y = torch.empty(lens.size, dtype=dt, device="cuda")
+        assert _csr.spmm_spmv(d, i, pt, lens.size, k, Bd, plan, C[1], xd, y)
+        yref = oracle.spmv(ptr, idx, rounded(data, dname), rounded(x, dname))
+        ysc = oracle.spmv_abs(ptr, idx, np.abs(rounded(data, dname)), np.abs(rounded(x, dname)))
+        _check(C[1], ref, scale, n, dname, "fused C")
+        assert_within(host(y).astype(np.float64), yref, spmv_error_bound(dname, yref, ysc, lens), "fused y")
+        # this matrix as A^T: dX = A^T dY with dY = B, values read through the identity permutation
+        perm = torch.arange(idx.size, dtype=torch.int32, device="cuda")
+        dX = torch.empty_like(C[0])
+        assert _csr.spmm_backward(d, perm, i, pt, k, lens.size, Bd, None, dX, None, plan)
+        _check(dX, ref, scale, n, dname, "dX")
+        assert plan.counters_clear()
+
+
 # ---------------------------------------------------------------- opt entry points / API contract
 
 def test_spmm_opt_entry_points_agree():
