@@ -36,16 +36,36 @@ namespace {
 // fused kernel of the batched step stays at 8: its persistent grid levels the
 // items itself (256 uneven matrices: 1.90 against 2.02 ms).
 constexpr int kSpmmWarps = 2;
+// Rows of at least this many bytes, made of whole 32-byte slices on 32-byte
+// boundaries, give each lane a 32-byte slice: half the lanes per row, so a warp
+// instruction loads, addresses and tests twice the nonzeros.  At 2 warps per
+// block (300,000 rows of Poisson(20)): bf16, 128 columns 205 -> 172 us; fp32,
+// 128 columns 364 -> 330 us, 32 columns 99 -> 92 us; fp64 64 columns on a
+// 300,000-row Zipf matrix 386 -> 337 us.  64-byte rows lose (fp32 68 -> 75 us:
+// teams of two lanes, and the wider sums at row ends), except in the fused
+// kernel, which also gathers x once per lane of a team (256 uneven matrices,
+// 16 columns: 1.90 -> 1.75 ms with two slices ahead; four: 2.00 ms).
+// Real types; compensated sums only in fp64 (64 columns 520 -> 472 us; fp32, 128
+// columns lose, 531 against 559 us, their pairs of sums spilling); the fused
+// kernel only in fp32.
+template <bool FUSED>
+constexpr int kSlice32Row = FUSED ? 64 : 128;
+template <int DT, bool COMP, bool FUSED>
+constexpr bool kSlice32 = FUSED ? DT == FSB_F32 && !COMP : !VT<DT>::kComplex && (!COMP || DT == FSB_F64);
 template <bool FUSED>
 constexpr int kTeamWarps = FUSED ? 8 : kSpmmWarps;
 constexpr int kSpmmBatch = 128;    // nonzeros staged per batch
 constexpr int kSpmmMaxCap = 64;    // row blocks hold < 2*cap <= kSpmmBatch nonzeros
-constexpr int kSpmmAhead = 4;      // B slices loaded ahead of the multiply-adds
+// B slices a team loads ahead of its sums: 4; 6 in one-team warps; 2 of 32
+// bytes in the fused kernel, whose x gathers and y sums need the registers
+constexpr int kSpmmAhead = 4, kOneTeamAhead = 6, kFused32Ahead = 2;
 template <int BYTES> struct RawT;
 template <> struct RawT<2> { using T = unsigned short; };
 template <> struct RawT<4> { using T = unsigned int; };
 template <> struct RawT<8> { using T = uint2; };
 template <> struct RawT<16> { using T = uint4; };
+struct Raw32 { uint32_t r[8]; };
+template <> struct RawT<32> { using T = Raw32; };
 
 // V consecutive elements starting at p; the first nv < V only when the slice
 // crosses column N (the rest read as zero).  ONCE: a streaming (evict-first)
@@ -70,14 +90,15 @@ __device__ __forceinline__ void load_slice(const S* p, int nv, S (&out)[V]) {
 
 // A lane's share of a team's column tile: P pieces of E consecutive elements,
 // a team's T lanes side by side in each piece, piece q of lane tl starting at
-// tile column (q * T + tl) * E.  Aligned rows take one 16-byte piece (P = 1).
+// tile column (q * T + tl) * E.  Aligned rows take one 16- or 32-byte piece
+// (P = 1, see kSlice32Row).
 // Other widths take pieces of one element or, where N, the leading dimensions
 // and the addresses allow, of 4 or 8 bytes; each piece lies wholly inside or
 // outside the N columns.
 template <typename S, int E, int P>
 struct Slice {
   static constexpr int V = E * P;
-  static constexpr bool kWhole = P == 1 && E * int(sizeof(S)) == 16;
+  static constexpr bool kWhole = P == 1 && E * int(sizeof(S)) >= 16;
   using Raw = typename RawT<E * int(sizeof(S))>::T;
   int off[P];  // this lane's first column of each piece, any valid column for pieces past N
   int nv;      // valid pieces
@@ -100,7 +121,14 @@ struct Slice {
                                 : static_cast<uint64_t>(row) * static_cast<uint64_t>(ldb));
 #pragma unroll
     for (int q = 0; q < P; ++q) {
-      const Raw w = __ldg(reinterpret_cast<const Raw*>(r + (kWhole ? 0 : off[q])));
+      Raw w;
+      if constexpr (sizeof(Raw) == 32)
+        asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=r"(w.r[0]), "=r"(w.r[1]), "=r"(w.r[2]), "=r"(w.r[3]), "=r"(w.r[4]), "=r"(w.r[5]), "=r"(w.r[6]),
+              "=r"(w.r[7])
+            : "l"(r));
+      else
+        w = __ldg(reinterpret_cast<const Raw*>(r + (kWhole ? 0 : off[q])));
       memcpy(&out[q * E], &w, sizeof(Raw));
     }
   }
@@ -111,7 +139,12 @@ struct Slice {
       if (q < nv) {
         Raw w;
         memcpy(&w, &v[q * E], sizeof(Raw));
-        __stcs(reinterpret_cast<Raw*>(row + off[q]), w);
+        if constexpr (sizeof(Raw) == 32)
+          asm volatile("st.global.cs.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(row + off[q]), "r"(w.r[0]),
+                       "r"(w.r[1]), "r"(w.r[2]), "r"(w.r[3]), "r"(w.r[4]), "r"(w.r[5]), "r"(w.r[6]), "r"(w.r[7])
+                       : "memory");
+        else
+          __stcs(reinterpret_cast<Raw*>(row + off[q]), w);
       }
   }
 };
@@ -424,21 +457,19 @@ constexpr int spmm_team_warp_smem_bytes() {
 }
 
 // Resident warps the register budget is sized for, in units of 8: 4 (64
-// registers) for plain sums of 2- and 4-byte values, 3 (85) for 8-byte values
-// and for compensated or fused sums, 2 for complex fp64.  More resident warps
-// keep more B rows in flight: wide rows measured up to 15 % faster at 4 units
-// with 4 slices ahead than at 3 with 6 ahead.  Three or four pieces per lane
-// spill at 64 registers: 80 against 87 us at 3 units (47 columns of fp32, a
-// 170,001-row Chung-Lu graph).
-template <int DT, bool COMP, bool FUSED, int P>
+// registers) for plain sums of 2- and 4-byte values, 3 (80) for 8-byte values,
+// for compensated or fused sums, for 32-byte slices (bf16, 128 columns: 172
+// against 195 us at 2.5 and 2 slices ahead in 242 us at 4) and for three or
+// four pieces per lane (80 against 87 us at 4: 47 columns of fp32, a
+// 170,001-row Chung-Lu graph); 2 for complex fp64 and 32-byte slices of fp64.
+template <int DT, bool COMP, bool FUSED, int E, int P>
 struct SpmmTeamWarps8 {
+  static constexpr bool k8 = DT == FSB_F64 || DT == FSB_C64;
+  static constexpr bool k32 = E * int(sizeof(typename VT<DT>::Store)) == 32;
   static constexpr int value =
-      (DT == FSB_C128) ? 2 : (!COMP && !FUSED && P < 3 && DT != FSB_F64 && DT != FSB_C64) ? 4 : 3;
+      DT == FSB_C128 ? 2 : k32 ? (k8 ? 2 : 3) : (!COMP && !FUSED && P < 3 && !k8) ? 4 : 3;
 };
 
-// B-row slices a team loads ahead of its sums in the row walk (KP): 4 for
-// teams narrower than the warp, 6 for 32-lane teams, whose warp walks its
-// rows alone and needs more of them in flight.
 template <int DT, bool COMP, int V>
 __device__ __forceinline__ void acc_shfl_add(SpmmAcc<DT, COMP, V>& a, int m) {
 #pragma unroll
@@ -729,7 +760,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
 }
 
 template <int DT, bool COMP, bool FUSED, int KP, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
-__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, P>::value * 8 / kTeamWarps<FUSED>)
+__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, E, P>::value * 8 / kTeamWarps<FUSED>)
 k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
             const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
             typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int T, int64_t tiles,
@@ -740,9 +771,9 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
   constexpr int V = E * P;
   using Acc = SpmmAcc<DT, COMP, V>;
   constexpr int kP = KP;
-  // the KP != 4 instantiation runs 32-lane teams only (one team per warp): a
+  // the KP = 6 instantiation runs 32-lane teams only (one team per warp): a
   // run's rows all end inside the team, so it has no scan and parks nothing
-  constexpr bool kOneTeam = KP != 4;
+  constexpr bool kOneTeam = KP == kOneTeamAhead;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -953,7 +984,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     }
     if constexpr (kCompLong<DT, COMP>) {
       if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
-        team_chunk<DT, (KP > kSpmmAhead ? 3 : 2), FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
+        team_chunk<DT, (KP == kOneTeamAhead ? 3 : 2), FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
                                                                    pstride, cps, x, y, sh_a, sh_c);
         continue;
       }
@@ -1325,12 +1356,12 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
                      void* C, int64_t ldc, const fsb_spmv_plan& plan, int T, int64_t tiles, cudaStream_t st,
                      const void* x = nullptr, void* y = nullptr) {
   using S = typename VT<DT>::Store;
-  constexpr bool kAligned = P == 1 && E * int(sizeof(S)) == 16;
+  constexpr bool kAligned = P == 1 && E * int(sizeof(S)) >= 16, k32 = E * int(sizeof(S)) == 32;
   const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kTeamWarps<FUSED>;
-  const int wide = (kAligned && !FUSED && T == 32) ? 1 : 0;
-  auto kern = k_spmm_team<DT, COMP, FUSED, 4, E, P>;
-  if constexpr (kAligned)
-    if (wide) kern = k_spmm_team<DT, COMP, FUSED, 6, E, P>;
+  const int wide = (kAligned && !k32 && !FUSED && T == 32) ? 1 : 0;
+  auto kern = k_spmm_team<DT, COMP, FUSED, FUSED && k32 ? kFused32Ahead : kSpmmAhead, E, P>;
+  if constexpr (kAligned && !k32 && !FUSED)
+    if (wide) kern = k_spmm_team<DT, COMP, FUSED, kOneTeamAhead, E, P>;
   if (smem > 48 * 1024) {  // opt in to the larger dynamic shared memory once per kernel and device
     static std::atomic<uint64_t> done[2];
     int dev = 0;
@@ -1381,6 +1412,14 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
   return FSB_OK;
 }
 
+// Whether the rows of B and C are whole slices of `bytes` bytes on such boundaries.
+template <typename S>
+bool spmm_whole_slices(int bytes, int64_t n, const void* B, int64_t ldb, const void* C, int64_t ldc) {
+  const int64_t v = bytes / int64_t(sizeof(S));
+  return n % v == 0 && ldb % v == 0 && ldc % v == 0 && reinterpret_cast<uintptr_t>(B) % bytes == 0 &&
+         reinterpret_cast<uintptr_t>(C) % bytes == 0;
+}
+
 // C = A B and y = A x in one launch: the team kernel with the fused y sums.
 // Real types, narrow aligned rows (the team conditions) and n < the slot
 // stride, so that y's long-row partial has a column of its own.
@@ -1392,10 +1431,16 @@ int spmm_spmv_fused(const void* data, const int32_t* idx, const int64_t* ptr, co
   if constexpr (VT<DT>::kComplex) {
     return FSB_ERR_UNSUPPORTED;
   } else {
-    if (!(n * int64_t(sizeof(S)) <= 256 && n % kVmax == 0 && ldb % kVmax == 0 && ldc % kVmax == 0 &&
-          reinterpret_cast<uintptr_t>(B) % 16 == 0 && reinterpret_cast<uintptr_t>(C) % 16 == 0 &&
-          n < spmm_pstride(n)))
+    if (!(n * int64_t(sizeof(S)) <= 256 && spmm_whole_slices<S>(16, n, B, ldb, C, ldc) && n < spmm_pstride(n)))
       return FSB_ERR_UNSUPPORTED;
+    if constexpr (kSlice32<DT, false, true>) {
+      if (!(plan.flags & FSB_SPMM_COMPENSATED) && n * int64_t(sizeof(S)) >= kSlice32Row<true> &&
+          spmm_whole_slices<S>(32, n, B, ldb, C, ldc)) {
+        int T = 1;
+        while (int64_t(T) * 2 * kVmax < n) T *= 2;
+        return spmm_launch_team<DT, false, true, 2 * kVmax>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, 1, st, x, y);
+      }
+    }
     int T = 1;
     while (int64_t(T) * kVmax < n) T *= 2;
     if (plan.flags & FSB_SPMM_COMPENSATED)
@@ -1474,11 +1519,14 @@ int spmm_dispatch(const void* data, const int32_t* idx, const int64_t* ptr, cons
                   int64_t n_cols, void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
   using S = typename VT<DT>::Store;
   constexpr int kVmax = 16 / int(sizeof(S));
-  // rows of whole, aligned 16-byte slices: teams of T lanes over column tiles
-  // of T * 16 bytes (spmm_team_tile_bytes)
-  if (n % kVmax == 0 && ldb % kVmax == 0 && ldc % kVmax == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(C) % 16 == 0 && ldb <= UINT32_MAX && n <= INT32_MAX) {
+  // rows of whole, aligned slices: teams of T lanes over column tiles of T
+  // slices (spmm_team_tile_bytes)
+  if (spmm_whole_slices<S>(16, n, B, ldb, C, ldc) && ldb <= UINT32_MAX && n <= INT32_MAX) {
     const int w = spmm_team_tile_bytes(n * int64_t(sizeof(S)), plan.tile_bytes);
+    if constexpr (kSlice32<DT, COMP, false>)
+      if (w >= kSlice32Row<false> && spmm_whole_slices<S>(32, n, B, ldb, C, ldc))
+        return spmm_launch_team<DT, COMP, false, 2 * kVmax>(data, idx, ptr, B, ldb, n, C, ldc, plan, w / 32,
+                                                            ceil_div(n, int64_t(w / 32) * 2 * kVmax), st);
     const int T = w / 16;
     return spmm_launch_team<DT, COMP>(data, idx, ptr, B, ldb, n, C, ldc, plan, T, ceil_div(n, int64_t(T) * kVmax),
                                       st);

@@ -384,6 +384,31 @@ def test_spmm_long_row_joins(dname, N):
         assert plan.counters_clear()
 
 
+@pytest.mark.parametrize("dname", ["float32", "bfloat16", "float64"])
+@pytest.mark.parametrize("width", [128, 160, 192, 288, 512, 544])
+@pytest.mark.parametrize("off", [0, 16])
+def test_spmm_32_byte_slices(dname, width, off):
+    """Rows of whole 32-byte slices from 128 bytes on (teams of 4 to 16 lanes, lanes past N, two
+    tiles), and the same widths 16 bytes off such boundaries: both kernels meet the bound."""
+    dt = TORCH_DT[dname]
+    s = torch.empty(0, dtype=dt).element_size()
+    N, gap = width // s, off // s
+    lens = np.array([0, 1, 2, 9, 33, 64, 0, 65, 257, 1500, 8] + [3] * 90 + [0, 40, 0], dtype=np.int64)
+    ptr = np.concatenate([[0], np.cumsum(lens)])
+    k = 2000
+    rng = np.random.Generator(np.random.PCG64(width))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int32)
+    data, B = rng.standard_normal(idx.size), rng.standard_normal((k, N))
+    Bw = torch.zeros(k * N + gap, dtype=dt, device="cuda")[gap:].view(k, N)
+    Bw.copy_(dev(B, dt))
+    plan = _csr.SpmmPlan(dev(ptr), lens.size, dt)
+    C = _csr.spmm(dev(data, dt), dev(idx), dev(ptr), lens.size, k, Bw, plan,
+                  torch.empty(lens.size, N, dtype=dt, device="cuda"))
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(data, dname), (lens.size, k), rounded(B, dname), "non")
+    _check(C, ref, scale, n, dname, f"{dname} {width} bytes + {off}")
+    assert plan.counters_clear()
+
+
 # ---------------------------------------------------------------- opt entry points / API contract
 
 def test_spmm_opt_entry_points_agree():
