@@ -10,8 +10,12 @@
 // together with a transpose butterfly (6 shuffles for 4 results instead of
 // 20).  Consecutive nonzeros mostly share a row, so the x slice is an L1 hit.
 //
-// That generic kernel serves every shape; rows of 5 to 64 aligned 16-byte
-// slices take the team kernel below, which caches the x row per team.
+// That generic kernel serves every shape; K-rows of up to 1,024 bytes in whole
+// pieces (sddmm_try_team) take the team kernel below, several nonzeros per warp
+// instruction, which keeps the x row per team.  (Narrow rows left most lanes of
+// the generic kernel idle, and rows off the 16-byte slices ran it too: fp32 on
+// a 300,000-node graph, 8 columns 342 -> 42 us, 16 columns 340 -> 60 us, 37
+// columns 416 -> 158 us.)
 //
 // Accumulation: fp32 for half / bfloat16 / fp32, fp64 for fp64 (fp64 for every
 // type with FSB_SDDMM_ACC64, which the reference's "acc64" variants select),
@@ -27,8 +31,14 @@
 namespace fsb {
 namespace {
 
-constexpr int kSddmmWarps = 8;
+// Warps per block.  2 rather than 8: a block's place is free when its last warp
+// ends (64 columns of fp32 on a 500,000-node graph: 311 against 361 us at 8).
+constexpr int kSddmmWarps = 2;
 constexpr int kSddmmGroup = 4;  // nonzeros reduced together
+// K-rows of at least this many bytes take 32-byte pieces where they can: half
+// the lanes per row and half the instructions per nonzero of 16-byte ones (64
+// columns of fp32 on that graph 441 -> 311 us; fp64, 32 columns 213 -> 180 us).
+constexpr int kSlice32 = 128;
 
 template <int BYTES> struct SRaw;
 template <> struct SRaw<2> { using T = unsigned short; };
@@ -138,56 +148,17 @@ k_sddmm_csr(const int32_t* __restrict__ row_ids, const int32_t* __restrict__ col
 }
 
 // ---------------------------------------------------------------------------
-// Fast path: teams of T lanes (8, 16 or 32) own 16-byte slices of a K-row,
-// TILES (1 or 2) slices per lane, so T * VW * TILES >= K.  A team walks U = 4
-// consecutive nonzeros per round; it keeps its current x row in registers as
-// fp32 and reloads it only when the row changes, so each nonzero costs one
-// 16-byte y load per lane.  The four dot products are reduced across the team
-// by a transpose butterfly: after the T/2 step a lane holds 2 items, after
-// T/4 one, then log2(T/4) plain steps.
+// Team kernel.  Teams of T lanes (2 to 32) own a K-row as P pieces of E
+// consecutive elements per lane, a team's lanes side by side in each piece.
+// A team walks U = 4 consecutive nonzeros per round with their y slices in
+// flight together, and keeps its current x row, loaded when the row changes
+// (holding the round's first and last row instead, loaded beside the y slices,
+// measured slower: 364 against 311 us below, its registers and branches cost
+// more than the wait).  The four
+// dot products are reduced across the team by a transpose butterfly: after the
+// T/2 step a lane holds 2 items, after T/4 one, then log2(T/4) plain steps.
 // ---------------------------------------------------------------------------
 constexpr int kTeamU = 4;
-
-template <typename S> struct Widen;
-template <> struct Widen<__nv_bfloat16> {
-  static constexpr int VW = 8;
-  __device__ __forceinline__ static void run(const uint4& w, float (&f)[8]) {
-    const unsigned u[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      f[2 * i] = __uint_as_float(u[i] << 16);
-      f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-    }
-  }
-};
-template <> struct Widen<__half> {
-  static constexpr int VW = 8;
-  __device__ __forceinline__ static void run(const uint4& w, float (&f)[8]) {
-    const unsigned u[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __half2 h;
-      memcpy(&h, &u[i], 4);
-      const float2 p = __half22float2(h);
-      f[2 * i] = p.x;
-      f[2 * i + 1] = p.y;
-    }
-  }
-};
-template <> struct Widen<float> {
-  static constexpr int VW = 4;
-  __device__ __forceinline__ static void run(const uint4& w, float (&f)[4]) {
-    f[0] = __uint_as_float(w.x); f[1] = __uint_as_float(w.y);
-    f[2] = __uint_as_float(w.z); f[3] = __uint_as_float(w.w);
-  }
-};
-template <> struct Widen<double> {
-  static constexpr int VW = 2;
-  __device__ __forceinline__ static void run(const uint4& w, double (&f)[2]) {
-    f[0] = __hiloint2double(int(w.y), int(w.x));
-    f[1] = __hiloint2double(int(w.w), int(w.z));
-  }
-};
 
 // acc += lo(x) * lo(y), then acc += hi(x) * hi(y) for two packed 16-bit
 // values each: sm_100a's mixed-precision fma.rn.f32.{bf16,f16} multiplies the
@@ -208,161 +179,217 @@ __device__ __forceinline__ float fma_pair16(unsigned xw, unsigned yw, float acc)
   return acc;
 }
 
-// 16-byte slice at p, or only its first nv elements (the rest zero).
-template <typename S>
-__device__ __forceinline__ uint4 slice16(const S* p, int nv) {
-  constexpr int VW = 16 / int(sizeof(S));
-  if (nv == VW) return __ldg(reinterpret_cast<const uint4*>(p));
-  S tmp[VW];
+// A lane's elements of a K-row: piece q is columns (q * T + tl) * E .. + E,
+// wholly inside K or (zero) outside it.
+template <typename S, int E, int P>
+struct KSlice {
+  static constexpr int V = E * P, kBytes = E * int(sizeof(S));
+  S v[V];
+  __device__ __forceinline__ void load(const S* __restrict__ row, int T, int tl, int k) {
 #pragma unroll
-  for (int j = 0; j < VW; ++j) {
-    if (j < nv) tmp[j] = p[j];
-    else memset(&tmp[j], 0, sizeof(S));
+    for (int q = 0; q < P; ++q) {
+      const int c = (q * T + tl) * E;
+      if (c < k) {
+        if constexpr (kBytes == 32) {
+          uint32_t r[8];
+          asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+              : "l"(row + c));
+          memcpy(&v[q * E], r, 32);
+        } else {
+          using Raw = typename SRaw<kBytes>::T;
+          const Raw r = __ldg(reinterpret_cast<const Raw*>(row + c));
+          memcpy(&v[q * E], &r, kBytes);
+        }
+      } else {
+        memset(&v[q * E], 0, kBytes);
+      }
+    }
   }
-  uint4 r;
-  memcpy(&r, tmp, 16);
-  return r;
-}
+  // the dot product of two slices, one chain in element order (pairs of 4-byte
+  // values: two chains, added)
+  template <typename R>
+  __device__ __forceinline__ R dot(const KSlice& o) const {
+    if constexpr (sizeof(S) == 2 && V % 2 == 0) {
+      float acc = 0.f;
+      unsigned a[V / 2], b[V / 2];
+      memcpy(a, v, sizeof(a));
+      memcpy(b, o.v, sizeof(b));
+#pragma unroll
+      for (int j = 0; j < V / 2; ++j) acc = fma_pair16<S>(a[j], b[j], acc);
+      return acc;
+    } else if constexpr (std::is_same<S, float>::value && V % 2 == 0) {
+      unsigned long long acc = 0;
+#pragma unroll
+      for (int j = 0; j < V; j += 2) {
+        unsigned long long a, b;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(v[j]), "f"(v[j + 1]));
+        asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(o.v[j]), "f"(o.v[j + 1]));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+      }
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+      return lo + hi;
+    } else {
+      R acc = R(0);
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc = fma(to_real(v[j]), to_real(o.v[j]), acc);
+      return acc;
+    }
+  }
+};
 
-template <int DT, int T, int TILES>
-__global__ void __launch_bounds__(kSddmmWarps * 32, TILES == 1 ? 4 : 3)
+// Blocks per SM the register budget is sized for, by a lane's bytes of a row: 80
+// registers for four 32-byte slices in flight (64 spill: 525 against 375 us on
+// the graph above, before the rest of this kernel's changes), else 64.
+constexpr int sddmm_blocks(int bytes) { return (bytes > 16 ? 24 : 32) / kSddmmWarps; }
+
+template <int DT, int T, int E, int P>
+__global__ void __launch_bounds__(kSddmmWarps * 32, sddmm_blocks(E * P * int(sizeof(typename VT<DT>::Store))))
 k_sddmm_team(const int32_t* __restrict__ row_ids, const int32_t* __restrict__ col, int64_t nnz,
              const typename VT<DT>::Store* __restrict__ x, int64_t ldx, const typename VT<DT>::Store* __restrict__ y,
-             int64_t ldy, int64_t k, const typename VT<DT>::Store* __restrict__ in, double alpha, double beta,
+             int64_t ldy, int k, const typename VT<DT>::Store* __restrict__ in, double alpha, double beta,
              typename VT<DT>::Store* __restrict__ out) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
-  using W = Widen<S>;
-  constexpr int VW = W::VW;
-  constexpr int G = 32 / T;                 // teams per warp
-  constexpr int PER_ROUND = G * kTeamU;     // nonzeros per warp round
-  static_assert(T >= 8 && T <= 32, "team size");
+  using Sl = KSlice<S, E, P>;
+  constexpr int G = 32 / T;                              // teams per warp
+  constexpr int kRound = G * kTeamU;                     // nonzeros per warp round
+  constexpr int kOwn = kRound > 32 ? kRound : 32, kW = kOwn / 32;  // nonzeros per warp
+  static_assert(T >= 2 && T <= 32, "team size");
   const int lane = threadIdx.x & 31;
   const int team = lane / T, tl = lane % T;
-  const int64_t base = (int64_t(blockIdx.x) * kSddmmWarps + (threadIdx.x >> 5)) * 32;
+  const int64_t base = (int64_t(blockIdx.x) * kSddmmWarps + (threadIdx.x >> 5)) * kOwn;
   if (base >= nnz) return;  // whole warp leaves together
-  const int cnt = nnz - base < 32 ? static_cast<int>(nnz - base) : 32;
-  int my_r = -1, my_c = 0;
-  if (lane < cnt) {
-    my_r = __ldcs(row_ids + base + lane);
-    my_c = __ldcs(col + base + lane);
-  }
-  int nvt[TILES];
-  int64_t off[TILES];
+  const int cnt = nnz - base < kOwn ? static_cast<int>(nnz - base) : kOwn;
+  int my_r[kW], my_c[kW];
 #pragma unroll
-  for (int t = 0; t < TILES; ++t) {
-    off[t] = (int64_t(t) * T + tl) * VW;
-    nvt[t] = static_cast<int>(k - off[t] >= VW ? int64_t(VW) : (k > off[t] ? k - off[t] : int64_t(0)));
+  for (int w = 0; w < kW; ++w) {  // past the end: the last nonzero again, computed and not written
+    const int i = min(w * 32 + lane, cnt - 1);
+    my_r[w] = __ldcs(row_ids + base + i);
+    my_c[w] = __ldcs(col + base + i);
   }
   const R a = static_cast<R>(alpha), b = static_cast<R>(beta);
-  // 16-bit values: x rows stay packed and multiply through fma_pair16
-  constexpr bool kMixed = sizeof(S) == 2;
-  int cur = -1;
-  R xf[TILES][VW];
-  uint4 xw[TILES];
-#pragma unroll
-  for (int t = 0; t < TILES; ++t) {
-    xw[t] = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-    for (int j = 0; j < VW; ++j) xf[t][j] = R(0);
-  }
+  Sl xs;
+  int cur = -1;  // the row that xs holds
 
-  for (int r0 = 0; r0 < cnt; r0 += PER_ROUND) {
+  for (int r0 = 0; r0 < cnt; r0 += kRound) {
     const int first = r0 + team * kTeamU;  // this team's items: first .. first+3
     int rq[kTeamU], cq[kTeamU];
 #pragma unroll
     for (int u = 0; u < kTeamU; ++u) {
-      rq[u] = __shfl_sync(0xffffffffu, my_r, (first + u) & 31);
-      cq[u] = __shfl_sync(0xffffffffu, my_c, (first + u) & 31);
-    }
-    uint4 yw[kTeamU][TILES];
+      const int src = (first + u) & 31;
+      rq[u] = __shfl_sync(0xffffffffu, my_r[0], src);
+      cq[u] = __shfl_sync(0xffffffffu, my_c[0], src);
 #pragma unroll
-    for (int u = 0; u < kTeamU; ++u) {
-      const bool valid = first + u < cnt;
-#pragma unroll
-      for (int t = 0; t < TILES; ++t)
-        yw[u][t] = slice16<S>(y + int64_t(cq[u]) * ldy + off[t], valid ? nvt[t] : 0);
-    }
-    R part[kTeamU];
-#pragma unroll
-    for (int u = 0; u < kTeamU; ++u) {
-      part[u] = R(0);
-      if (first + u < cnt) {
-        if (rq[u] != cur) {  // uniform inside the team
-          cur = rq[u];
-#pragma unroll
-          for (int t = 0; t < TILES; ++t) {
-            if constexpr (kMixed) xw[t] = slice16<S>(x + int64_t(cur) * ldx + off[t], nvt[t]);
-            else W::run(slice16<S>(x + int64_t(cur) * ldx + off[t], nvt[t]), xf[t]);
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < TILES; ++t) {
-          if constexpr (kMixed) {
-            part[u] = fma_pair16<S>(xw[t].x, yw[u][t].x, part[u]);
-            part[u] = fma_pair16<S>(xw[t].y, yw[u][t].y, part[u]);
-            part[u] = fma_pair16<S>(xw[t].z, yw[u][t].z, part[u]);
-            part[u] = fma_pair16<S>(xw[t].w, yw[u][t].w, part[u]);
-          } else {
-            R yf[VW];
-            W::run(yw[u][t], yf);
-#pragma unroll
-            for (int j = 0; j < VW; ++j) part[u] = fma(xf[t][j], yf[j], part[u]);
-          }
+      for (int w = 1; w < kW; ++w) {
+        const int r = __shfl_sync(0xffffffffu, my_r[w], src), c = __shfl_sync(0xffffffffu, my_c[w], src);
+        if (((first + u) >> 5) == w) {
+          rq[u] = r;
+          cq[u] = c;
         }
       }
     }
+    Sl ys[kTeamU];
+#pragma unroll
+    for (int u = 0; u < kTeamU; ++u) ys[u].load(y + int64_t(cq[u]) * ldy, T, tl, k);
+    R part[kTeamU];
+#pragma unroll
+    for (int u = 0; u < kTeamU; ++u) {
+      if (rq[u] != cur) {  // uniform inside the team
+        cur = rq[u];
+        xs.load(x + int64_t(cur) * ldx, T, tl, k);
+      }
+      part[u] = xs.template dot<R>(ys[u]);
+    }
     // transpose butterfly inside the team
     constexpr int H = T / 2, Q = T / 4;
-    const bool hb = tl & H, qb = tl & Q;
+    const bool hb = tl & H, qb = Q > 0 && (tl & Q);
     R s0 = hb ? part[2] : part[0], s1 = hb ? part[3] : part[1];
-    const R o0 = hb ? part[0] : part[2], o1 = hb ? part[1] : part[3];
-    s0 += __shfl_xor_sync(0xffffffffu, o0, H);
-    s1 += __shfl_xor_sync(0xffffffffu, o1, H);
-    R v = qb ? s1 : s0;
-    v += __shfl_xor_sync(0xffffffffu, qb ? s0 : s1, Q);
+    s0 += __shfl_xor_sync(0xffffffffu, hb ? part[0] : part[2], H);
+    s1 += __shfl_xor_sync(0xffffffffu, hb ? part[1] : part[3], H);
+    auto put = [&](int item, R v) {
+      if (item < cnt) {
+        const int64_t p = base + item;
+        R res = v * a;
+        if (in) res += to_real(in[p]) * b;
+        out[p] = sddmm_out(res, out);
+      }
+    };
+    if constexpr (Q == 0) {  // two lanes: two finished items each
+      put(first + (hb ? 2 : 0), s0);
+      put(first + (hb ? 3 : 1), s1);
+    } else {
+      R v = qb ? s1 : s0;
+      v += __shfl_xor_sync(0xffffffffu, qb ? s0 : s1, Q);
 #pragma unroll
-    for (int m = Q / 2; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-    const int item = first + (hb ? 2 : 0) + (qb ? 1 : 0);
-    if ((tl & (Q - 1)) == 0 && item < cnt) {
-      const int64_t p = base + item;
-      R res = v * a;
-      if (in) res += to_real(in[p]) * b;
-      out[p] = sddmm_out(res, out);
+      for (int m = Q / 2; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+      if ((tl & (Q - 1)) == 0) put(first + (hb ? 2 : 0) + (qb ? 1 : 0), v);
     }
   }
 }
 
-template <int DT, int T, int TILES>
+template <int DT, int T, int E, int P>
 int sddmm_launch_team(const int32_t* row_ids, const int32_t* col, int64_t nnz, const void* x, int64_t ldx,
                       const void* y, int64_t ldy, int64_t k, const void* in, double alpha, double beta, void* out,
                       cudaStream_t st) {
   using S = typename VT<DT>::Store;
-  const int64_t blocks = ceil_div(ceil_div(nnz, 32), kSddmmWarps);
+  constexpr int kOwn = 32 / T * kTeamU > 32 ? 32 / T * kTeamU : 32;
+  const int64_t blocks = ceil_div(ceil_div(nnz, kOwn), kSddmmWarps);
   if (blocks > INT32_MAX) return FSB_ERR_UNSUPPORTED;
-  k_sddmm_team<DT, T, TILES><<<(unsigned)blocks, kSddmmWarps * 32, 0, st>>>(
-      row_ids, col, nnz, static_cast<const S*>(x), ldx, static_cast<const S*>(y), ldy, k, static_cast<const S*>(in),
-      alpha, beta, static_cast<S*>(out));
+  k_sddmm_team<DT, T, E, P><<<(unsigned)blocks, kSddmmWarps * 32, 0, st>>>(
+      row_ids, col, nnz, static_cast<const S*>(x), ldx, static_cast<const S*>(y), ldy, static_cast<int>(k),
+      static_cast<const S*>(in), alpha, beta, static_cast<S*>(out));
   FSB_LAUNCH_CHECK();
   return FSB_OK;
 }
 
-// Fast path when x / y rows are 16-byte aligned and K fits two 16-byte
-// slices per lane of a 32-lane team; returns 1 when it launched (rc set).
+// A row as `pieces` pieces of E elements, P per lane.
+template <int DT, int E, int P, int T = 32>
+int sddmm_launch_pieces(int pieces, const int32_t* row_ids, const int32_t* col, int64_t nnz, const void* x,
+                        int64_t ldx, const void* y, int64_t ldy, int64_t k, const void* in, double alpha, double beta,
+                        void* out, cudaStream_t st) {
+  if constexpr (T > 2)
+    if (pieces <= T / 2 * P)
+      return sddmm_launch_pieces<DT, E, P, T / 2>(pieces, row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out,
+                                                  st);
+  return sddmm_launch_team<DT, T, E, P>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
+}
+
+// The team kernel where a K-row is at most 1,024 bytes of whole pieces: returns
+// 1 when it launched (rc set).  Pieces are the widest of 32 (rows of at least
+// kSlice32 bytes), 16, 8, 4 and 2 bytes that divide K, the leading dimensions
+// and the addresses.
 template <int DT>
 int sddmm_try_team(const int32_t* row_ids, const int32_t* col, int64_t nnz, const void* x, int64_t ldx,
                    const void* y, int64_t ldy, int64_t k, const void* in, double alpha, double beta, void* out,
                    int* rc, cudaStream_t st) {
   using S = typename VT<DT>::Store;
-  constexpr int VW = 16 / int(sizeof(S));
-  if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(y) % 16 || ldx % VW || ldy % VW) return 0;
-  const int64_t slices = ceil_div(k, VW);  // 16-byte slices per row
-  if (slices < 5 || slices > 64) return 0;
-  if (slices <= 8) *rc = sddmm_launch_team<DT, 8, 1>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
-  else if (slices <= 16) *rc = sddmm_launch_team<DT, 16, 1>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
-  else if (slices <= 32) *rc = sddmm_launch_team<DT, 32, 1>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
-  else *rc = sddmm_launch_team<DT, 32, 2>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
-  return 1;
+  constexpr int s = int(sizeof(S));
+  auto whole = [&](int bytes) {
+    const int e = bytes / s;
+    return k % e == 0 && ldx % e == 0 && ldy % e == 0 && reinterpret_cast<uintptr_t>(x) % bytes == 0 &&
+           reinterpret_cast<uintptr_t>(y) % bytes == 0;
+  };
+  auto run = [&](auto e, auto p) {
+    constexpr int E = decltype(e)::value, P = decltype(p)::value;
+    if (k > int64_t(32) * P * E) return 0;
+    *rc = sddmm_launch_pieces<DT, E, P>(static_cast<int>(k / E), row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta,
+                                        out, st);
+    return 1;
+  };
+#define FSB_I(n) std::integral_constant<int, (n)>()
+  if (k < 1) return 0;
+  if (k * s >= kSlice32 && whole(32)) return run(FSB_I(32 / s), FSB_I(1));
+  if (whole(16)) return k * s <= 512 ? run(FSB_I(16 / s), FSB_I(1)) : run(FSB_I(16 / s), FSB_I(2));
+  if constexpr (s <= 8)
+    if (whole(8)) return run(FSB_I(8 / s), FSB_I(2)) || run(FSB_I(8 / s), FSB_I(4));
+  if constexpr (s <= 4)
+    if (whole(4)) return run(FSB_I(4 / s), FSB_I(4));
+  if constexpr (s <= 2)
+    if (whole(2)) return run(FSB_I(1), FSB_I(4));
+#undef FSB_I
+  return 0;
 }
 
 template <int DT, int V, bool ACC64, bool OUT64>

@@ -60,6 +60,38 @@ def test_sddmm_native_dtypes_and_widths(dname, K):
     assert_within(host(out).astype(np.float64), ref, plain_error_bound(dname, ref, scale, K), f"{dname} K={K}")
 
 
+@pytest.mark.parametrize("dname", ["bfloat16", "float32", "float64"])
+@pytest.mark.parametrize("K", [1, 2, 3, 4, 5, 8, 12, 16, 20, 33, 47, 48, 72, 96, 127, 129, 256, 257, 512])
+@pytest.mark.parametrize("gap", [0, 1, 8])
+def test_sddmm_piece_widths(dname, K, gap):
+    """Every piece size and team width: widths, leading dimensions (K + gap) and addresses on and
+    off the 32-, 16-, 8- and 4-byte boundaries, rows that change inside a team's four nonzeros, a
+    last partial warp; and an infinite y entry in its own column's products only."""
+    lens = [0, 1, 1, 1, 2, 3, 0, 0, 4, 5, 31, 32, 33, 200, 0, 7] + [1, 0, 2] * 40
+    indptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    n_cols = 90
+    rng = np.random.Generator(np.random.PCG64(K))
+    indices = np.concatenate([np.sort(rng.integers(0, n_cols, n)) for n in lens]).astype(np.int32)
+    dt = TORCH_DT[dname]
+    x_np, y_np = rng.standard_normal((len(lens), K)), rng.standard_normal((n_cols, K))
+
+    def wide(a):  # `gap` elements past an allocation's start, rows `gap` apart
+        buf = torch.zeros(gap + a.shape[0] * (K + gap), dtype=dt, device="cuda")[gap:]
+        v = buf.view(a.shape[0], K + gap)[:, :K]
+        v.copy_(dev(a, dt))
+        return v
+
+    x, y = wide(x_np), wide(y_np)
+    row_ids = dm._build_row_ids(dev(indptr))
+    out = torch.empty(indices.size, dtype=dt, device="cuda")
+    dm._native_sddmm(row_ids, dev(indices), x, y, None, 1.0, 0.0, out)
+    ref, scale = _oracle(indptr, indices, rounded(x_np, dname), rounded(y_np, dname), None, 1.0, 0.0)
+    assert_within(host(out).astype(np.float64), ref, plain_error_bound(dname, ref, scale, K), f"{dname} K={K}")
+    y[17, 0] = float("inf")
+    dm._native_sddmm(row_ids, dev(indices), x, y, None, 1.0, 0.0, out)
+    assert np.array_equal(~np.isfinite(host(out)), indices == 17)
+
+
 def test_sddmm_row_ids_match_reference_rule():
     c = workloads.zipf_csr(n=30_000, seed=21)
     for ptr_dt in (torch.int64, torch.int32):
