@@ -132,6 +132,19 @@ struct Slice {
       memcpy(&out[q * E], &w, sizeof(Raw));
     }
   }
+  // slice of the row at `row`, read once: a streaming (evict-first) load
+  __device__ __forceinline__ void load_once(const S* __restrict__ row, S (&out)[V]) const {
+    static_assert(kWhole, "whole slices");
+    Raw w;
+    if constexpr (sizeof(Raw) == 32)
+      asm("ld.global.cs.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+          : "=r"(w.r[0]), "=r"(w.r[1]), "=r"(w.r[2]), "=r"(w.r[3]), "=r"(w.r[4]), "=r"(w.r[5]), "=r"(w.r[6]),
+            "=r"(w.r[7])
+          : "l"(row + off[0]));
+    else
+      w = __ldcs(reinterpret_cast<const Raw*>(row + off[0]));
+    memcpy(out, &w, sizeof(Raw));
+  }
   // streaming (evict-first) stores: the output is written once
   __device__ __forceinline__ void store(S* __restrict__ row, const S (&v)[V]) const {
 #pragma unroll
@@ -284,9 +297,14 @@ struct SpmmAcc {
   }
 };
 
-// resident warps of the backward, in units of 8
-template <int DT>
-struct SpmmBwdWarps8 { static constexpr int value = (DT == FSB_C128) ? 2 : (DT == FSB_F64 || DT == FSB_C64) ? 3 : 4; };
+// Blocks per SM that the backward's register budget is sized for: 10 (96
+// registers) with 32-byte slices, 12 (80) with 16-byte ones.  Training step on a
+// 500,000-node Chung-Lu graph, bf16, 128 columns: 1087 us at 96 registers, 1080
+// at 128, 1616 at 80 (spills); 16-byte slices 1160 at 80, 1320 at 72.
+template <int DT, int E>
+struct SpmmBwdBlocks {
+  static constexpr int value = E * int(sizeof(typename VT<DT>::Store)) == 32 ? 10 : 12;
+};
 
 // Gather of x for the fused y sums: L2-only.
 template <typename T> __device__ __forceinline__ T ld_gather(const T* p) { return __ldcg(p); }
@@ -405,8 +423,8 @@ __device__ __forceinline__ void stage_offsets(int32_t* sh_off, const int64_t* __
 // Rows of more than this many nonzeros accumulate compensated in the types
 // whose sums run in fp32 (f16, bf16, f32), whatever the plan's flags: their
 // sums are the long ones.  Shorter rows keep the plan's accumulation.  The
-// forward kernels use Dot2 (blocked in the team kernel), the backward fp64
-// sums of the exact products.
+// forward kernel uses Dot2, blocked Dot2 or fp64 sums (ChunkAcc), the backward
+// fp64 sums of the exact products.
 constexpr int64_t kCompensateAbove = 1024;
 template <int DT, bool COMP>
 constexpr bool kCompLong = !COMP && (DT == FSB_F16 || DT == FSB_BF16 || DT == FSB_F32);
@@ -571,10 +589,9 @@ __device__ __forceinline__ void acc_shfl_add(WideAcc<DT, V>& a, int m) { a.shfl_
 // accumulator, so the error is at most gamma_(KA+1) * sum|a||b| plus
 // the final rounding whatever the row length (the chunk and team partials
 // are combined compensated as well); 3 fp64 sums of the exact products
-// (WideAcc), far inside that bound.  Modes 2 and 3 serve the same rows of
-// the fp32-accumulated types: 3 in the one-team kernel, where it measured
-// faster (fp32, 128 columns: 2.21 against 2.25 ms), 2 elsewhere (fp64 sums
-// cost 4-5 % on 256-byte rows).
+// (WideAcc), far inside that bound.  The fp32-accumulated types' rows over
+// kCompensateAbove nonzeros use 3 in column tiles of 512 bytes, 2 in narrower
+// ones (fp64 sums cost 3-5 % on 256-byte rows) and 1 in widths off the slices.
 template <int DT, int MODE, int V>
 struct ChunkAcc;
 template <int DT, int V>
@@ -975,22 +992,30 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     const fsb_spmv_unit* ud = plan.units + nb + (item - n_groups);
     const int32_t nch = __ldg(&ud->n_chunks);
     // rows of more than kCompensateAbove nonzeros sum compensated in the
-    // fp32-accumulated types, partials and all (blocked Dot2, or fp64 sums
-    // in the one-team kernel)
+    // fp32-accumulated types, partials and all (see ChunkAcc)
+    auto chunk = [&](auto mode) {
+      team_chunk<DT, decltype(mode)::value, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
+                                                             pstride, cps, x, y, sh_a, sh_c);
+    };
     if constexpr (COMP) {
-      team_chunk<DT, 1, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl, pstride, cps, x, y, sh_a,
-                                         sh_c);
+      chunk(std::integral_constant<int, 1>());
       continue;
     }
     if constexpr (kCompLong<DT, COMP>) {
       if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
-        team_chunk<DT, (KP == kOneTeamAhead ? 3 : 2), FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
-                                                                   pstride, cps, x, y, sh_a, sh_c);
+        constexpr bool k32 = E * int(sizeof(S)) == 32;
+        if constexpr (!Slice<S, E, P>::kWhole) {
+          chunk(std::integral_constant<int, 1>());
+        } else if constexpr (kOneTeam) {
+          chunk(std::integral_constant<int, 3>());
+        } else {
+          if (k32 && !FUSED && T == 16) chunk(std::integral_constant<int, k32 && !FUSED ? 3 : 2>());
+          else chunk(std::integral_constant<int, 2>());
+        }
         continue;
       }
     }
-    team_chunk<DT, 0, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl, pstride, cps, x, y, sh_a,
-                                       sh_c);
+    chunk(std::integral_constant<int, 0>());
   }
 }
 
@@ -1001,23 +1026,61 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
 //   dX[c]   += vals[p] * dY[r]      A^T dY, laid out as in k_spmm_team
 //   dvals[p] = <dY[r], X[c]>        the SDDMM of dY and X on A's pattern
 // The dY row slice of each nonzero is gathered once and serves both sums; A's
-// values are read through perm (no transposed copy), and X[c] is loaded once
-// per row of A^T.  Teams of T lanes (T * V >= n, T <= 32) own 16-byte column
-// slices.  The dot products of each group of slices loaded ahead reduce across
-// the team by a transpose butterfly (log2 of the group size halving steps, then
-// plain xor steps) in a fixed order; the lanes left holding a finished product
-// write it.  With DV false dvals is not formed (dX only).  X is read with
-// streaming loads and dX written with streaming stores, which keep more of the
-// gathered dY rows in L2 (measured 0.5 % faster).
+// values are read through perm (no transposed copy).  Work is cut as in
+// k_spmm_team: teams of T lanes take equal shares of the nonzeros of a run of
+// up to 4 units, whatever the row lengths (one team per row left the teams of
+// short rows waiting for the longest of theirs, and single units paid the
+// perm -> value -> dY chain every 50 nonzeros: bf16 training step on a
+// 500,000-node Chung-Lu graph, 128 columns, 1232 -> 1087 us with 32-byte slices;
+// 200,000 nodes, 64 columns 190 -> 146 us; fp32, 64 columns 210 -> 187 us; fp32,
+// 128 columns on the large graph is bound by its dY traffic, 1.75 ms either
+// way).  A team holds the X slice of
+// its current row and loads the next row's beside the dY slices of the step in
+// which the row changes.  The dot products of a step reduce across the team by
+// a transpose butterfly (log2 of the step's size halving steps, then plain xor
+// steps) in a fixed order; the lanes left holding a finished product write it.
+// With DV false dvals is not formed (dX only).  X is read with streaming loads
+// and dX written with streaming stores, which keep more of the gathered dY
+// rows in L2 (measured 0.5 % faster).
 // ---------------------------------------------------------------------------
-// dY row slices loaded ahead of the sums: 8 for 4- and 8-byte values, 4 for
-// half / bfloat16, whose 8-wide slices and widened products spill at 8
-template <int DT>
-struct BwdAhead { static constexpr int value = (DT == FSB_F16 || DT == FSB_BF16) ? 4 : 8; };
+constexpr int kBwdAhead = 4;  // dY row slices loaded ahead of the sums
 
+// Per-warp slice: staged values, columns, positions in A and run-local row
+// offsets, then (16-byte aligned) one parked accumulator per lane.
 template <typename S>
+constexpr int spmm_bwd_park_offset() {
+  return (spmm_team_vals_bytes<S>() + 2 * kRowStage * 4 + (kRowRows + 1) * 4 + 15) & ~15;
+}
+template <int DT, int V>
 constexpr int spmm_bwd_warp_smem_bytes() {
-  return (kSpmmBatch * (int(sizeof(S)) + 8) + (kSpmmMaxCap + 1) * 4 + 15) & ~15;
+  return spmm_bwd_park_offset<typename VT<DT>::Store>() + 32 * int(sizeof(SpmmAcc<DT, false, V>));
+}
+
+// Stages values (through perm), columns and positions of nonzeros
+// [s0, s0 + cnt), cnt <= kRowStage.
+template <typename S>
+__device__ __forceinline__ void stage_perm(S* sh_a, int32_t* sh_c, int32_t* sh_p, const S* __restrict__ vals,
+                                           const int32_t* __restrict__ perm, const int32_t* __restrict__ col,
+                                           int64_t s0, int cnt, int lane) {
+  for (int k = lane; k < cnt; k += 32) cp_async<4>(sh_c + k, col + s0 + k);
+  constexpr int kU = 4;
+  for (int k0 = lane; k0 < cnt; k0 += 32 * kU) {
+    int32_t q[kU];
+    S v[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + 32 * u < cnt) q[u] = ld_once(perm + s0 + k0 + 32 * u);
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + 32 * u < cnt) v[u] = vals[q[u]];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + 32 * u < cnt) {
+        sh_p[k0 + 32 * u] = q[u];
+        sh_a[k0 + 32 * u] = v[u];
+      }
+  }
+  cp_async_wait_all();
 }
 
 // Reduces d[0..M) of every lane across the T lanes of its team.  On return the
@@ -1058,8 +1121,6 @@ __device__ __forceinline__ void ffma2x(float& c0, float& c1, float a0, float a1,
   asm("mov.b64 {%0, %1}, %2;" : "=f"(c0), "=f"(c1) : "l"(cc));
 }
 
-// Per-lane partial dot products of the kA dY slices with this lane's X slice
-// (already widened to R); fp32 sums run as two packed halves added at the end.
 // (c0, c1) += (lo(x) * lo(b), hi(x) * hi(b)) for packed 16-bit x and b, one
 // rounding each (see fma_mixed2).
 template <typename S>
@@ -1075,30 +1136,27 @@ __device__ __forceinline__ void fma_mixed2x(float& c0, float& c1, unsigned x, un
   }
 }
 
-// xs: the same X slice as xf, unwidened (16-bit values multiply from it).
-template <typename S, typename R, int KA, int V>
-__device__ __forceinline__ void bwd_dots(const S (&bv)[KA][V], const R (&xf)[V], const S (&xs)[V], R (&d)[KA]) {
+// Partial dot product of one dY slice with this lane's X slice.
+template <typename S, typename R, int V>
+__device__ __forceinline__ R slice_dot(const S (&b)[V], const S (&x)[V]) {
+  if constexpr (sizeof(S) == 2 && V % 2 == 0) {
+    unsigned xw[V / 2], bw[V / 2];
+    memcpy(xw, x, sizeof(xw));
+    memcpy(bw, b, sizeof(bw));
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-  for (int u = 0; u < KA; ++u) {
-    if constexpr (sizeof(S) == 2 && V % 2 == 0) {
-      unsigned xw[V / 2], bw[V / 2];
-      memcpy(xw, xs, sizeof(xw));
-      memcpy(bw, bv[u], sizeof(bw));
-      float s0 = 0.f, s1 = 0.f;
+    for (int j = 0; j < V / 2; ++j) fma_mixed2x<S>(s0, s1, xw[j], bw[j]);
+    return s0 + s1;
+  } else if constexpr (std::is_same<R, float>::value && V % 2 == 0) {
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-      for (int j = 0; j < V / 2; ++j) fma_mixed2x<S>(s0, s1, xw[j], bw[j]);
-      d[u] = s0 + s1;
-    } else if constexpr (std::is_same<R, float>::value && V % 2 == 0) {
-      float s0 = 0.f, s1 = 0.f;
+    for (int j = 0; j < V; j += 2) ffma2x(s0, s1, to_real(b[j]), to_real(b[j + 1]), to_real(x[j]), to_real(x[j + 1]));
+    return s0 + s1;
+  } else {
+    R s = R(0);
 #pragma unroll
-      for (int j = 0; j < V; j += 2) ffma2x(s0, s1, to_real(bv[u][j]), to_real(bv[u][j + 1]), xf[j], xf[j + 1]);
-      d[u] = s0 + s1;
-    } else {
-      R s = R(0);
-#pragma unroll
-      for (int j = 0; j < V; ++j) s = fma(to_real(bv[u][j]), xf[j], s);
-      d[u] = s;
-    }
+    for (int j = 0; j < V; ++j) s = fma(to_real(b[j]), to_real(x[j]), s);
+    return s;
   }
 }
 
@@ -1118,8 +1176,8 @@ __device__ __forceinline__ void bwd_put_dots(R (&d)[KA], int base, int stride, i
   }
 }
 
-template <int DT, bool DV>
-__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmBwdWarps8<DT>::value * 8 / kSpmmWarps)
+template <int DT, bool DV, int E>
+__global__ void __launch_bounds__(kSpmmWarps * 32, SpmmBwdBlocks<DT, E>::value)
 k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __restrict__ perm,
            const int32_t* __restrict__ col, const int64_t* __restrict__ ptr,
            const typename VT<DT>::Store* __restrict__ dY, int64_t lddy, int64_t n,
@@ -1128,148 +1186,233 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
            int64_t cps) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
-  constexpr int V = 16 / int(sizeof(S));
+  constexpr int V = E, kP = kBwdAhead;
   using Acc = SpmmAcc<DT, false, V>;
-  constexpr int kER = Acc::kNC * 2;
-  constexpr int kA = BwdAhead<DT>::value;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t unit = int64_t(blockIdx.x) * kSpmmWarps + warp;
-  if (unit >= plan.n_units) return;  // whole warp leaves together
   const int G = 32 / T, team = lane / T, tl = lane % T;
-  const int64_t c0 = int64_t(tl) * V;
-  const int nv = c0 + V <= n ? V : 0;  // n is a multiple of V
-
-  unsigned char* wbase = smem_raw + warp * spmm_bwd_warp_smem_bytes<S>();
+  unsigned char* wbase = smem_raw + warp * spmm_bwd_warp_smem_bytes<DT, V>();
   S* sh_a = reinterpret_cast<S*>(wbase);
-  int32_t* sh_c = reinterpret_cast<int32_t*>(wbase + kSpmmBatch * sizeof(S));
-  int32_t* sh_p = sh_c + kSpmmBatch;
-  int32_t* sh_off = sh_p + kSpmmBatch;
+  int32_t* sh_c = reinterpret_cast<int32_t*>(wbase + spmm_team_vals_bytes<S>());
+  int32_t* sh_p = sh_c + kRowStage;
+  int32_t* sh_off = sh_p + kRowStage;
+  Acc* sh_park = reinterpret_cast<Acc*>(wbase + spmm_bwd_park_offset<S>()) + lane;
 
-  const fsb_spmv_unit* ud = plan.units + unit;
-  const int64_t s0 = __ldg(&ud->nnz_begin), s1 = __ldg(&ud->nnz_end);
-  const int32_t row = __ldg(&ud->row), tag = __ldg(&ud->tag);
+  const int64_t nb = plan.n_block_units;
+  const uint32_t n_groups = static_cast<uint32_t>(ceil_div(nb, kRowUnits));
+  const uint32_t item = blockIdx.x * kSpmmWarps + warp;
+  if (item >= n_groups + static_cast<uint32_t>(plan.n_units - nb)) return;  // whole warp leaves together
+  Slice<S, E, 1> sl;  // lanes past N load column 0, take no part in the dots and store nothing
+  sl.set(0, T, tl, n);
+  const S* Bl = sl.base(dY);
+  auto load_x = [&](int64_t row, S (&out)[V]) { sl.load_once(X + row * ldx, out); };
+  auto dot = [&](const S (&b)[V], const S (&x)[V]) { return sl.nv > 0 ? slice_dot<S, R, V>(b, x) : R(0); };
 
-  // stages a batch of <= kSpmmBatch nonzeros (a strided loop: unrolling the
-  // loads ahead costs registers that the gathers below need)
-  auto stage = [&](int64_t from, int cnt) {
-    for (int k = lane; k < cnt; k += 32) {
-      const int32_t p = ld_once(perm + from + k);
-      sh_p[k] = p;
-      sh_a[k] = vals[p];
-      sh_c[k] = ld_once(col + from + k);
+  if (item < n_groups) {
+    // ------------------------------------------------------------ row group
+    const int64_t ua = int64_t(item) * kRowUnits;
+    const int nu = static_cast<int>(nb - ua < kRowUnits ? nb - ua : int64_t(kRowUnits));
+    int64_t d_s0 = 0, d_s1 = 0;
+    int32_t d_row = 0, d_tag = 0;
+    if (lane < nu) {
+      const int4* p = reinterpret_cast<const int4*>(plan.units + ua + lane);
+      const int4 a = __ldg(p), b = __ldg(p + 1);
+      d_s0 = (int64_t)(uint32_t)a.x | ((int64_t)a.y << 32);
+      d_s1 = (int64_t)(uint32_t)a.z | ((int64_t)a.w << 32);
+      d_row = b.x;
+      d_tag = b.y;
     }
-  };
-  if (tag >= 0) {
-    // ------------------------------------------------------------ row block
-    const int nr = tag - row;
-    const int cnt = static_cast<int>(s1 - s0);
-    stage_offsets<kSpmmMaxCap>(sh_off, ptr, row, nr, s0, lane);
-    stage(s0, cnt);
-    __syncwarp();
-    for (int i0 = 0; i0 < nr; i0 += G) {
-      const int i = i0 + team;
-      const bool has = i < nr;
-      const int b = has ? sh_off[i] : 0;
-      const int len = has ? sh_off[i + 1] - b : 0;
-      int maxlen = len;
-      for (int m = T; m < 32; m <<= 1) maxlen = max(maxlen, __shfl_xor_sync(0xffffffffu, maxlen, m));
-      R xf[V];
-      S xs[V];
-      if constexpr (DV) {
-        load_slice<S, V, true>(X + (int64_t(row) + (has ? i : 0)) * ldx + c0, len > 0 ? nv : 0, xs);
-#pragma unroll
-        for (int j = 0; j < V; ++j) xf[j] = to_real(xs[j]);
+    int u = 0;
+    while (u < nu) {  // runs of units whose rows join up, as in k_spmm_team
+      const int32_t r0 = __shfl_sync(0xffffffffu, d_row, u);
+      const int64_t s0 = __shfl_sync(0xffffffffu, d_s0, u);
+      int32_t r1 = __shfl_sync(0xffffffffu, d_tag, u);
+      int64_t s1 = __shfl_sync(0xffffffffu, d_s1, u);
+      int v = u + 1;
+      for (; v < nu; ++v) {
+        if (__shfl_sync(0xffffffffu, d_row, v) != r1) break;
+        r1 = __shfl_sync(0xffffffffu, d_tag, v);
+        s1 = __shfl_sync(0xffffffffu, d_s1, v);
       }
+      u = v;
+      const int nr = r1 - r0;
+      const int cnt = static_cast<int>(s1 - s0);
+      __syncwarp();  // the staging slice of the previous run is free
+      stage_offsets<kRowRows>(sh_off, ptr, r0, nr, s0, lane);
+      stage_perm<S>(sh_a, sh_c, sh_p, vals, perm, col, s0, cnt, lane);
+      __syncwarp();
+      auto put_row = [&](const Acc& a, int r) {
+        if (sl.nv > 0) {
+          S o[V];
+          a.result(o);
+          sl.store(dX + (int64_t(r0) + r) * lddx, o);
+        }
+      };
+      for (int i0 = 0; i0 < nr; i0 += 32) {  // empty rows get zero slices (one team each)
+        const int i = i0 + lane;
+        unsigned m = __ballot_sync(0xffffffffu, i < nr && sh_off[i] == sh_off[i + 1]);
+        for (int q = 0; m; ++q) {
+          const int b = __ffs(m) - 1;
+          m &= m - 1;
+          if (q % G == team) {
+            Acc z;
+            z.zero();
+            put_row(z, i0 + b);
+          }
+        }
+      }
+      if (cnt == 0) continue;
+
+      // team g takes nonzeros [jb, je) of the run (see k_spmm_team)
+      const int per = (cnt + G - 1) / G;
+      const int jb = min(team * per, cnt), je = min(jb + per, cnt);
       Acc acc;
       acc.zero();
-      for (int k = 0; k < maxlen; k += kA) {
-        S bv[kA][V];
-#pragma unroll
-        for (int u = 0; u < kA; ++u) {
-          const bool ok = k + u < len;
-          load_slice<S, V>(dY + int64_t(sh_c[ok ? b + k + u : 0]) * lddy + c0, ok ? nv : 0, bv[u]);
+      int cur = 0;  // the row of nonzero jb: the last row whose offset is <= jb
+      {
+        int lo = 0, hi = nr - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (sh_off[mid] <= jb) lo = mid; else hi = mid - 1;
         }
-#pragma unroll
-        for (int u = 0; u < kA; ++u)
-          if (k + u < len) acc.add(sh_a[b + k + u], bv[u]);
-        if constexpr (DV) {
-          R d[kA];
-          bwd_dots<S, R, kA, V>(bv, xf, xs, d);
-          bwd_put_dots<S, R, kA>(d, b + k, 1, b + len, T, tl, sh_p, dvals);
-        }
+        cur = lo;
       }
-      if (has && nv > 0) {
-        S o[V];
-        acc.result(o);
-        store_slice<S, V, true>(dX + (int64_t(row) + i) * lddx + c0, nv, o);
+      int next_end = jb < je ? sh_off[cur + 1] : cnt;
+      bool open_start = jb < je && sh_off[cur] < jb;
+      int park_row = -1;
+      S xa[V], xb[V];
+      if constexpr (DV) {
+        if (jb < je) load_x(int64_t(r0) + cur, xa);
+      }
+      // every team takes the same number of steps: the butterflies are warp-wide
+      for (int t = 0; t < per; t += kP) {
+        const int j0 = jb + t;
+        S bv[kP][V];
+        R d[kP];
+#pragma unroll
+        for (int q = 0; q < kP; ++q)  // past je: some nonzero, loaded and not summed
+          sl.load(Bl, static_cast<uint32_t>(sh_c[min(j0 + q, max(je - 1, 0))]), lddy, bv[q]);
+        int xrow = -1;
+        if constexpr (DV) {
+          if (next_end < je && next_end < j0 + kP) {  // the row changes in this step
+            xrow = cur + 1;
+            while (sh_off[xrow + 1] == next_end) ++xrow;
+            load_x(int64_t(r0) + xrow, xb);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < kP; ++q) {
+          const int j = j0 + q;
+          if constexpr (DV) d[q] = R(0);
+          if (j < je) {
+            if (j == next_end) {  // row cur ended before nonzero j
+              if (open_start) {
+                *sh_park = acc;  // finished after the scan
+                park_row = cur;
+                open_start = false;
+              } else {
+                put_row(acc, cur);
+              }
+              acc.zero();
+              do {
+                ++cur;
+                next_end = sh_off[cur + 1];
+              } while (next_end == j);
+              if constexpr (DV) {
+                if (cur == xrow) memcpy(xa, xb, sizeof(xa));
+                else load_x(int64_t(r0) + cur, xa);
+              }
+            }
+            acc.add(sh_a[j], bv[q]);
+            if constexpr (DV) d[q] = dot(bv[q], xa);
+          }
+        }
+        if constexpr (DV) bwd_put_dots<S, R, kP>(d, j0, 1, je, T, tl, sh_p, dvals);
+      }
+      // inclusive segmented scan of the open-ended partials over the teams
+      const bool open_end = jb < je && next_end > je;  // row cur goes on in later teams
+      const int key = open_end ? cur : -1;
+      Acc sc = acc;
+      if (!open_end) sc.zero();
+      for (int o = 1; o < G; o <<= 1) {
+        Acc other;
+        acc_shfl_up(sc, other, o * T);
+        const int okey = __shfl_up_sync(0xffffffffu, key, o * T);
+        if (team >= o && key >= 0 && okey == key) acc_combine(sc, other);
+      }
+      Acc carry;
+      acc_shfl_up(sc, carry, T);
+      if (park_row >= 0) {
+        Acc f = *sh_park;
+        acc_combine(f, carry);
+        put_row(f, park_row);
+      }
+      if (jb < je && !open_end) {
+        if (open_start) acc_combine(acc, carry);
+        put_row(acc, cur);
       }
     }
     return;
   }
 
   // ------------------------------------------------------------ long-row chunk
+  const fsb_spmv_unit* ud = plan.units + nb + (item - n_groups);
+  const int64_t s0 = __ldg(&ud->nnz_begin), s1 = __ldg(&ud->nnz_end);
+  const int32_t row = __ldg(&ud->row), tag = __ldg(&ud->tag);
   const int32_t nch = __ldg(&ud->n_chunks), slot = __ldg(&ud->slot);
-  R xf[V];
+  const int64_t c0 = int64_t(tl) * V;  // this lane's place in a slot's partials
   S xs[V];
-  if constexpr (DV) {
-    load_slice<S, V, true>(X + int64_t(row) * ldx + c0, nv, xs);
-#pragma unroll
-    for (int j = 0; j < V; ++j) xf[j] = to_real(xs[j]);
-  }
-  // WIDE (rows over kCompensateAbove nonzeros, see kCompLong): fp64 sums of
-  // the exact products (WideAcc) with kA / 2 dY slices in flight, which keeps
-  // the kernel within the plain path's registers (measured on the 500,000-node
-  // Chung-Lu graph, 128 columns: fp32 no slower than plain sums, bf16 3.5 %
-  // slower; Dot2 sums cost 3.5 % / 8 %); else plain sums
+  if constexpr (DV) load_x(row, xs);
+  // WIDE (rows over kCompensateAbove nonzeros, see kCompLong): fp64 sums of the
+  // exact products; else plain sums
   auto run_chunk = [&](auto wide) {
-    constexpr bool kWide = decltype(wide)::value;
-    using A2 = typename std::conditional<kWide, WideAcc<DT, V>, Acc>::type;
-    constexpr int kAc = kWide ? kA / 2 : kA;
+    using A2 = typename std::conditional<decltype(wide)::value, WideAcc<DT, V>, Acc>::type;
+    constexpr int kER = A2::kNC * 2;
     A2 acc;
     acc.zero();
-    for (int64_t b0 = s0; b0 < s1; b0 += kSpmmBatch) {
-      const int cnt = static_cast<int>(s1 - b0 < kSpmmBatch ? s1 - b0 : int64_t(kSpmmBatch));
+    for (int64_t b0 = s0; b0 < s1; b0 += kRowStage) {
+      const int cnt = static_cast<int>(s1 - b0 < kRowStage ? s1 - b0 : int64_t(kRowStage));
       __syncwarp();
-      stage(b0, cnt);
+      stage_perm<S>(sh_a, sh_c, sh_p, vals, perm, col, b0, cnt, lane);
       __syncwarp();
-      for (int k = 0; k < cnt; k += kAc * G) {
-        S bv[kAc][V];
+      for (int k = 0; k < cnt; k += kP * G) {
+        S bv[kP][V];
+        R d[kP];
 #pragma unroll
-        for (int u = 0; u < kAc; ++u) {
-          const int kk = k + u * G + team;
-          load_slice<S, V>(dY + int64_t(sh_c[kk < cnt ? kk : 0]) * lddy + c0, kk < cnt ? nv : 0, bv[u]);
+        for (int q = 0; q < kP; ++q) {
+          const int kk = k + q * G + team;
+          sl.load(Bl, static_cast<uint32_t>(sh_c[kk < cnt ? kk : cnt - 1]), lddy, bv[q]);
         }
 #pragma unroll
-        for (int u = 0; u < kAc; ++u) {
-          const int kk = k + u * G + team;
-          if (kk < cnt) acc.add(sh_a[kk], bv[u]);
+        for (int q = 0; q < kP; ++q) {
+          const int kk = k + q * G + team;
+          if (kk < cnt) acc.add(sh_a[kk], bv[q]);
+          if constexpr (DV) d[q] = dot(bv[q], xs);
         }
-        if constexpr (DV) {
-          R d[kAc];
-          bwd_dots<S, R, kAc, V>(bv, xf, xs, d);
-          bwd_put_dots<S, R, kAc>(d, k + team, G, cnt, T, tl, sh_p, dvals);
-        }
+        if constexpr (DV) bwd_put_dots<S, R, kP>(d, k + team, G, cnt, T, tl, sh_p, dvals);
       }
     }
     for (int m = T; m < 32; m <<= 1) acc_shfl_add(acc, m);  // every team now holds the chunk's sum
-    if (nch == 1) {
-      if (team == 0 && nv > 0) {
+    auto put = [&](const A2& a) {
+      if (team == 0 && sl.nv > 0) {
         S o[V];
-        acc.result(o);
-        store_slice<S, V, true>(dX + int64_t(row) * lddx + c0, nv, o);
+        a.result(o);
+        sl.store(dX + int64_t(row) * lddx, o);
       }
+    };
+    if (nch == 1) {
+      put(acc);
       return;
     }
     R* part = static_cast<R*>(plan.partials);
     const int64_t first = int64_t(slot) + (tag + 1);
     if (team == 0) acc.store_partial(part + (int64_t(slot) * pstride + c0) * kER);
-    auto total = [&](int64_t from, int64_t step, int count) {
+    auto total = [&](int64_t from, int64_t stride, int count) {
       A2 fin;
       fin.zero();
 #pragma unroll 4
-      for (int c = team; c < count; c += G) fin.add_partial(part + ((from + c * step) * pstride + c0) * kER);
+      for (int c = team; c < count; c += G) fin.add_partial(part + ((from + c * stride) * pstride + c0) * kER);
       for (int m = T; m < 32; m <<= 1) acc_shfl_add(fin, m);
       return fin;
     };
@@ -1280,12 +1423,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
       if (team == 0) g.store_partial(part + (join.group_slot * pstride + c0) * kER);
     }
     if (!join_ticket(plan.counters + first * cps, join.members, lane)) return;
-    const A2 fin = total(first, join.step, join.members);
-    if (team == 0 && nv > 0) {
-      S o[V];
-      fin.result(o);
-      store_slice<S, V, true>(dX + int64_t(row) * lddx + c0, nv, o);
-    }
+    put(total(first, join.step, join.members));
   };
   if constexpr (kCompLong<DT, false>) {
     if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
@@ -1463,26 +1601,33 @@ int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, con
     return FSB_ERR_UNSUPPORTED;
   } else {
     auto a16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-    if (!(n * int64_t(sizeof(S)) <= 512 && n % kVmax == 0 && lddy % kVmax == 0 && lddx % kVmax == 0 && a16(dY) &&
-          a16(dX) && (!dvals || (ldx % kVmax == 0 && a16(X)))) ||
-        (plan.flags & FSB_SPMM_COMPENSATED))
+    auto whole = [&](int bytes) {
+      return spmm_whole_slices<S>(bytes, n, dY, lddy, dX, lddx) &&
+             (!dvals || (ldx * int64_t(sizeof(S)) % bytes == 0 && reinterpret_cast<uintptr_t>(X) % bytes == 0));
+    };
+    if (n * int64_t(sizeof(S)) > 512 || lddy > UINT32_MAX || !whole(16) || (plan.flags & FSB_SPMM_COMPENSATED))
       return FSB_ERR_UNSUPPORTED;
-    int T = 1;
-    while (int64_t(T) * kVmax < n) T *= 2;
-    const int64_t blocks = ceil_div(plan.n_units, kSpmmWarps);
-    const size_t smem = size_t(spmm_bwd_warp_smem_bytes<S>()) * kSpmmWarps;
-    const S* v = static_cast<const S*>(vals);
-    if (dvals) {
-      k_spmm_bwd<DT, true><<<(unsigned)blocks, kSpmmWarps * 32, smem, st>>>(
-          v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, static_cast<const S*>(X), ldx,
-          static_cast<S*>(dX), lddx, static_cast<S*>(dvals), plan, T, spmm_pstride(n), spmm_cps<DT>(n));
-    } else {
-      k_spmm_bwd<DT, false><<<(unsigned)blocks, kSpmmWarps * 32, smem, st>>>(
-          v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, nullptr, 0, static_cast<S*>(dX), lddx, nullptr,
-          plan, T, spmm_pstride(n), spmm_cps<DT>(n));
-    }
-    FSB_LAUNCH_CHECK();
-    return FSB_OK;
+    auto run = [&](auto e) {
+      constexpr int E = decltype(e)::value;
+      int T = 1;
+      while (int64_t(T) * E < n) T *= 2;
+      const int64_t items = ceil_div(plan.n_block_units, kRowUnits) + (plan.n_units - plan.n_block_units);
+      const unsigned blocks = (unsigned)ceil_div(items, kSpmmWarps);
+      const size_t smem = size_t(spmm_bwd_warp_smem_bytes<DT, E>()) * kSpmmWarps;
+      const S* v = static_cast<const S*>(vals);
+      if (dvals)
+        k_spmm_bwd<DT, true, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
+            v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, static_cast<const S*>(X), ldx,
+            static_cast<S*>(dX), lddx, static_cast<S*>(dvals), plan, T, spmm_pstride(n), spmm_cps<DT>(n));
+      else
+        k_spmm_bwd<DT, false, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
+            v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, nullptr, 0, static_cast<S*>(dX), lddx, nullptr,
+            plan, T, spmm_pstride(n), spmm_cps<DT>(n));
+      FSB_LAUNCH_CHECK();
+      return int(FSB_OK);
+    };
+    if (n * int64_t(sizeof(S)) >= kSlice32Row<false> && whole(32)) return run(std::integral_constant<int, 2 * kVmax>());
+    return run(std::integral_constant<int, kVmax>());
   }
 }
 

@@ -144,3 +144,34 @@ def test_autograd_takes_one_launch_path(monkeypatch):
     assert calls == [True]
     _check("float32", (indptr, indices, host(vals).astype(np.float64), (800, 300)), host(X).astype(np.float64),
            host(G).astype(np.float64), X.grad, vals.grad, 16)
+
+
+@pytest.mark.parametrize("dname,n", [("float32", 16), ("float32", 40), ("float32", 72), ("float32", 104),
+                                    ("bfloat16", 80), ("bfloat16", 144), ("float64", 20)])
+def test_backward_row_changes_and_idle_lanes(dname, n):
+    """A^T rows of one to three nonzeros (the row changes several times in one step of a team),
+    empty ones between, one of several chunks; widths that leave lanes of a team past the last
+    column, with 16- and 32-byte slices.  An infinite dY entry reaches its own row's products and
+    the dX rows of its columns only."""
+    dt = TORCH[dname]
+    n_rows, n_cols = 900, 2600
+    rng = np.random.default_rng(n)
+    rows = [np.unique(np.concatenate([[2599], rng.integers(0, 650, 4) * 4])) for _ in range(n_rows)]
+    indptr = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int64)
+    indices = np.concatenate(rows).astype(np.int32)
+    data = rng.uniform(0.5, 1.0, indices.size)
+    vals = dev(data, dt)
+    p = fs.prepare_spmm_csr_autograd(vals, dev(indices), dev(indptr), (n_rows, n_cols))
+    X, dY = dev(rng.standard_normal((n_cols, n)), dt), dev(rng.standard_normal((n_rows, n)), dt)
+    dX, dvals = torch.empty(n_cols, n, dtype=dt, device="cuda"), torch.empty_like(vals)
+    args = (vals, p.perm32, p.t_indices, p.t_indptr, n_rows, n_cols)
+    assert _csr.spmm_backward(*args, dY, X, dX, dvals, p.t_plan)
+    mat = (indptr, indices, host(vals).astype(np.float64), (n_rows, n_cols))
+    _check(dname, mat, host(X).astype(np.float64), host(dY).astype(np.float64), dX, dvals, n)
+    assert p.t_plan.n_slots > 0 and p.t_plan.counters_clear()
+    dY[451, 0] = float("inf")
+    assert _csr.spmm_backward(*args, dY, X, dX, dvals, p.t_plan)
+    own = np.repeat(np.arange(n_rows), np.diff(indptr)) == 451
+    assert np.array_equal(~np.isfinite(host(dvals)), own)
+    bad = ~np.isfinite(host(dX))
+    assert np.array_equal(np.nonzero(bad.any(1))[0], np.sort(indices[own])) and not bad[:, 1:].any()
