@@ -72,6 +72,8 @@ _SIGNATURES = {
     "fsb_version": (_c_int, []),
     "fsb_status_string": (ctypes.c_char_p, [_c_int]),
     "fsb_csr_inspect": (_c_int, [_c_ptr, _c_int, _c_ptr, _c_int, _c_i64, _c_i64, _c_ptr, _c_ptr]),
+    "fsb_spmm_plan_order_workspace_bytes": (_c_i64, [_c_i64]),
+    "fsb_spmm_plan_order": (_c_int, [_c_ptr, _c_i64, _c_ptr, _c_i64, _c_i64, _c_ptr, _c_i64, _c_ptr]),
     "fsb_csr_bucketize_workspace_bytes": (_c_i64, [_c_i64, _c_int]),
     "fsb_csr_bucketize": (
         _c_int,

@@ -177,6 +177,86 @@ static int spmv_plan_build_impl(const PT* ptr, int64_t n_rows, int64_t cap, int6
   return FSB_OK;
 }
 
+// ---------------------------------------------------------------------------
+// SpMM: long-row chunks in column order.  A chunk of a long row covers a range
+// of columns (they are sorted within a row), so chunks listed by their first
+// column gather from one moving window of B, which stays in L2; listed by row
+// they gather from all of B at once.  1024 windows of n_cols / 1024 columns;
+// the order inside a window is left open: it moves work between warps, and
+// each chunk's sum and slot stay the same.  Where the columns are skewed the
+// chunks keep their order: a graph's hub columns would be hit by every warp at
+// once (bf16 training step on a 500,000-node Chung-Lu graph, 128 columns: 1086 ->
+// 1150 us).  On a 1 M-row power-law matrix, 128 columns: fp32 2.17 -> 1.94 ms,
+// bf16 1.32 -> 1.25 ms.
+// ---------------------------------------------------------------------------
+constexpr int kOrderWindows = 1024;
+
+__device__ __forceinline__ int order_window(const int32_t* idx, const fsb_spmv_unit& u, int64_t n_cols) {
+  const int64_t c = __ldg(idx + u.nnz_begin);
+  return static_cast<int>(c * kOrderWindows / n_cols);
+}
+
+// counts[0, 1024): chunks per window; counts[1024, 2048): the same without the
+// first chunks of rows, which all begin near column 0
+__global__ void k_order_count(const int32_t* idx, const fsb_spmv_unit* units, int64_t n, int64_t n_cols,
+                              int32_t* counts) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const fsb_spmv_unit u = units[i];
+  const int w = order_window(idx, u, n_cols);
+  atomicAdd(counts + w, 1);
+  if (u.tag < -1) atomicAdd(counts + kOrderWindows + w, 1);
+}
+
+// one block of kOrderWindows threads: counts -> first places; counts[1024] = 1
+// when the order is left alone: fewer than 1,024 later chunks (nothing to gain),
+// or skewed columns, a 64th of them with over 3 times its share of the later
+// chunks (uniform columns on 1 M power-law rows: 1.2 times; Chung-Lu graph: 5.2)
+__global__ void k_order_places(int32_t* counts) {
+  __shared__ int32_t warp_sum[32], later_max[32], later_sum[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int32_t mine = counts[t], later = counts[kOrderWindows + t];
+  int32_t v = mine, ls = later;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t up = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += up;
+  }
+  for (int o = 1; o < 16; o <<= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);  // 16 windows: a 64th
+  const int32_t other = __shfl_xor_sync(0xffffffffu, ls, 16);
+  int32_t lm = max(ls, other);
+  ls += other;
+  if (lane == 31) {
+    warp_sum[w] = v;
+    later_max[w] = lm;
+    later_sum[w] = ls;
+  }
+  __syncthreads();
+  if (w == 0) {
+    int32_t s = warp_sum[lane];
+    lm = later_max[lane];
+    ls = later_sum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t up = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += up;
+      lm = max(lm, __shfl_xor_sync(0xffffffffu, lm, o));
+      ls += __shfl_xor_sync(0xffffffffu, ls, o);
+    }
+    warp_sum[lane] = s;
+    if (lane == 0) counts[kOrderWindows] = ls < 1024 || int64_t(lm) * 64 > int64_t(ls) * 3;
+  }
+  __syncthreads();
+  counts[t] = v - mine + (w > 0 ? warp_sum[w - 1] : 0);
+}
+
+__global__ void k_order_place(const int32_t* idx, const fsb_spmv_unit* units, int64_t n, int64_t n_cols,
+                              int32_t* places, fsb_spmv_unit* out) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const fsb_spmv_unit u = units[i];
+  const int64_t at = places[kOrderWindows] ? i : atomicAdd(places + order_window(idx, u, n_cols), 1);
+  out[at] = u;
+}
+
 __global__ void k_copy_totals(const int64_t* src, int64_t* dst, int n) {
   if (threadIdx.x < n) dst[threadIdx.x] = src[threadIdx.x];
 }
@@ -421,6 +501,40 @@ int fsb_spmv_plan_build(const void* indptr, int ptr_is_64, int64_t n_rows, int32
                                 units, st);
   return spmv_plan_build_impl(static_cast<const int32_t*>(indptr), n_rows, cap, chunk_nnz, ws, seg_row0, seg_unit0,
                               units, st);
+}
+
+int64_t fsb_spmm_plan_order_workspace_bytes(int64_t n_chunks) {
+  return n_chunks < 0 ? -1 : 2 * kOrderWindows * int64_t(sizeof(int32_t)) + n_chunks * int64_t(sizeof(fsb_spmv_unit));
+}
+
+int fsb_spmm_plan_order(const int32_t* indices, int64_t n_cols, fsb_spmv_unit* units, int64_t n_block_units,
+                        int64_t n_units, void* workspace, int64_t workspace_bytes, void* stream) {
+  if (n_block_units < 0 || n_units < n_block_units) return FSB_ERR_INVALID_ARG;
+  const int64_t n = n_units - n_block_units;
+  if (n == 0) return FSB_OK;
+  if (!indices || !units || !workspace || n_cols < 1) return FSB_ERR_INVALID_ARG;
+  if (n_units >= INT32_MAX) return FSB_ERR_UNSUPPORTED;
+  if (workspace_bytes < fsb_spmm_plan_order_workspace_bytes(n)) return FSB_ERR_WORKSPACE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  int32_t* counts = static_cast<int32_t*>(workspace);
+  fsb_spmv_unit* out = reinterpret_cast<fsb_spmv_unit*>(counts + 2 * kOrderWindows);
+  fsb_spmv_unit* chunks = units + n_block_units;
+  const unsigned blocks = (unsigned)ceil_div(n, 256);
+  if (cudaMemsetAsync(counts, 0, 2 * kOrderWindows * sizeof(int32_t), st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return FSB_ERR_CUDA;
+  }
+  k_order_count<<<blocks, 256, 0, st>>>(indices, chunks, n, n_cols, counts);
+  FSB_LAUNCH_CHECK();
+  k_order_places<<<1, kOrderWindows, 0, st>>>(counts);
+  FSB_LAUNCH_CHECK();
+  k_order_place<<<blocks, 256, 0, st>>>(indices, chunks, n, n_cols, counts, out);
+  FSB_LAUNCH_CHECK();
+  if (cudaMemcpyAsync(chunks, out, n * sizeof(fsb_spmv_unit), cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return FSB_ERR_CUDA;
+  }
+  return FSB_OK;
 }
 
 int64_t fsb_csr_bucketize_workspace_bytes(int64_t n_rows, int n_buckets) {

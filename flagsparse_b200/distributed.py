@@ -115,7 +115,7 @@ class ShardedCsr:
         if self._spmm is None:
             data, ind, ptr, n_rows, n_cols, _rl, _mx = _prepare_spmm_csr_matrix(
                 self.data, self.indices, self.indptr, self.local_shape)
-            self._spmm = (data, ind, ptr, _csr.SpmmPlan(ptr, n_rows, data.dtype))
+            self._spmm = (data, ind, ptr, _csr.SpmmPlan(ptr, n_rows, data.dtype, indices=ind, n_cols=n_cols))
         return self._spmm
 
     def spmv(self, x, gather=False, out=None):

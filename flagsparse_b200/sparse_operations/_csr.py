@@ -239,14 +239,32 @@ class SpmmPlan:
     plus long-row scratch sized per dense width N (allocated once per N and
     reused; fsb_spmm_csr leaves the tickets zero after every call)."""
 
-    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None):
+    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None, indices=None, n_cols=0):
         lib = nat.lib()
         code = nat.dtype_code(dtype)
         self.dtype = dtype
         cap = int(lib.fsb_spmm_default_cap(code)) if cap is None else int(cap)
         chunk_nnz = int(lib.fsb_spmm_default_chunk(code)) if chunk_nnz is None else int(chunk_nnz)
         self.plan = NativeSpmvPlan(indptr, n_rows, dtype, cap=cap, chunk_nnz=chunk_nnz, scratch=False)
+        if indices is not None and n_cols > self.ORDER_ABOVE_COLS and self.plan.n_slots > 0:
+            self._order_chunks(indices, n_cols)
         self._scratch = {}  # n -> (partials, counters, SpmvPlan struct)
+
+    # Chunks are put in column order where a B of the widest column tile (512 bytes)
+    # is larger than the 126 MB L2; a smaller B stays there in any order.
+    ORDER_ABOVE_COLS = (126 << 20) // 512
+
+    def _order_chunks(self, indices, n_cols):
+        lib = nat.lib()
+        p = self.plan
+        n = p.n_units - p.n_block_units
+        ws_bytes = int(lib.fsb_spmm_plan_order_workspace_bytes(n))
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=p.units.device)
+        nat.check(
+            lib.fsb_spmm_plan_order(nat.ptr(indices), int(n_cols), nat.ptr(p.units), p.n_block_units, p.n_units,
+                                    nat.ptr(ws), ws_bytes, nat.stream_of(p.units.device)),
+            "fsb_spmm_plan_order",
+        )
 
     @property
     def n_units(self):

@@ -50,8 +50,8 @@ class PreparedCsrSpmmAutograd:
             self.perm = torch.empty(0, dtype=torch.int64, device=indices.device)
         # the one-launch backward reads A's values through an int32 permutation
         self.perm32 = self.perm.to(torch.int32) if 0 < self.nnz < 2**31 else None
-        self.plan = _csr.SpmmPlan(indptr, self.n_rows, dtype)
-        self.t_plan = _csr.SpmmPlan(self.t_indptr, self.n_cols, dtype)
+        self.plan = _csr.SpmmPlan(indptr, self.n_rows, dtype, indices=indices, n_cols=self.n_cols)
+        self.t_plan = _csr.SpmmPlan(self.t_indptr, self.n_cols, dtype, indices=self.t_indices, n_cols=self.n_rows)
 
     @property
     def row_ids(self):

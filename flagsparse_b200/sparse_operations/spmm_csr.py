@@ -362,8 +362,8 @@ def _native_spmm_into(data, kernel_indices, kernel_indptr, n_rows, n_cols, B, pl
     return _csr.spmm(data, kernel_indices, kernel_indptr, n_rows, n_cols, B, plan, out, compensated=compensated)
 
 
-def _spmm_plan(kernel_indptr, n_rows, dtype):
-    return _csr.SpmmPlan(kernel_indptr, n_rows, dtype)
+def _spmm_plan(kernel_indices, kernel_indptr, shape, dtype):
+    return _csr.SpmmPlan(kernel_indptr, int(shape[0]), dtype, indices=kernel_indices, n_cols=int(shape[1]))
 
 
 def _row_major_out(out, n_rows, n, dtype, device):
@@ -448,7 +448,7 @@ def flagsparse_spmm_csr(
         torch.cuda.synchronize()
         if _spmm_op_transposes(op_code):
             symbolic_ms = (time.perf_counter() - t0) * 1000.0
-    plan = _spmm_plan(kernel_indptr, n_rows, data.dtype)
+    plan = _spmm_plan(kernel_indices, kernel_indptr, (n_rows, n_cols), data.dtype)
     if max_segments is not None or block_nnz is not None:
         if max_row_nnz is None:
             max_row_nnz = int((kernel_indptr[1:] - kernel_indptr[:-1]).max().item()) if n_rows > 0 else 0
@@ -660,7 +660,7 @@ def _route_native(prepared, op_name, timing=False):
             _normalize_spmm_op(op_name),
         )
         route = _spmm_csr_route_from_materialized(prepared, data, indices, indptr, shape, op_name)
-    plan = _spmm_plan(route.kernel_indptr, route.n_rows, route.data.dtype)
+    plan = _spmm_plan(route.kernel_indices, route.kernel_indptr, route.shape, route.data.dtype)
     prepared._native[op_name] = (route, plan)
     ms = None
     if timing:
@@ -932,7 +932,7 @@ class PreparedCsrSpmmOpt:
 
     def native_plan(self):
         if self._native is None:
-            self._native = _spmm_plan(self.kernel_indptr, self.n_rows, self.data.dtype)
+            self._native = _spmm_plan(self.kernel_indices, self.kernel_indptr, self.shape, self.data.dtype)
         return self._native
 
 

@@ -61,7 +61,7 @@ class PreparedCsrSpmmOptAlg2:
 
     def native_plan(self):
         if self._native is None:
-            self._native = _spmm_plan(self.kernel_indptr, self.n_rows, self.data.dtype)
+            self._native = _spmm_plan(self.kernel_indices, self.kernel_indptr, self.shape, self.data.dtype)
         return self._native
 
 

@@ -215,6 +215,15 @@ FSB_API int fsb_spmv_plan_build(const void* indptr, int ptr_is_64, int64_t n_row
                         int32_t chunk_nnz, const void* workspace, int64_t workspace_bytes,
                         int32_t* seg_row0, int32_t* seg_unit0, fsb_spmv_unit* units, void* stream);
 
+/* Reorders a plan's long-row chunks, units[n_block_units, n_units), by the
+ * column of each chunk's first nonzero, so that SpMM chunks in flight together
+ * gather neighbouring rows of B.  The products stay bitwise the same.
+ * `indices` int32 in [0, n_cols); workspace 8-byte aligned, of
+ * fsb_spmm_plan_order_workspace_bytes(n_units - n_block_units) bytes. */
+FSB_API int64_t fsb_spmm_plan_order_workspace_bytes(int64_t n_chunks);
+FSB_API int fsb_spmm_plan_order(const int32_t* indices, int64_t n_cols, fsb_spmv_unit* units, int64_t n_block_units,
+                                int64_t n_units, void* workspace, int64_t workspace_bytes, void* stream);
+
 FSB_API int fsb_spmv_csr(int dtype, const void* data, const void* indices, int idx_is_64,
                  const void* indptr, int ptr_is_64, int64_t n_rows, int64_t n_cols,
                  const void* x, void* y, const fsb_spmv_plan* plan, void* stream);

@@ -409,6 +409,37 @@ def test_spmm_32_byte_slices(dname, width, off):
     assert plan.counters_clear()
 
 
+@pytest.mark.parametrize("skewed", [False, True])
+def test_spmm_chunk_order(skewed, monkeypatch):
+    """Long-row chunks in column order: the units stay the same set, row blocks and (with skewed
+    columns) every chunk in place; later chunks otherwise follow their columns' 1,024 windows.
+    Products are bitwise those of the plan in row order."""
+    n_rows, k, long = 700, 5000, 260
+    rng = np.random.Generator(np.random.PCG64(7))
+    lens = np.where(np.arange(n_rows) % 2 == 0, rng.integers(0, 60, n_rows), 0)
+    lens[rng.choice(n_rows, long, replace=False)] = rng.integers(1000, 2500, long)
+    w = np.arange(1, k + 1) ** -1.5 if skewed else np.ones(k)
+    cols = [np.sort(rng.choice(k, n, replace=False, p=w / w.sum())) for n in lens]
+    idx = dev(np.concatenate(cols).astype(np.int32))
+    ptr = dev(np.concatenate([[0], np.cumsum(lens)]).astype(np.int64))
+    data = torch.randn(idx.numel(), device="cuda")
+    B = torch.randn(k, 64, device="cuda")
+    plain = _csr.SpmmPlan(ptr, n_rows, torch.float32, indices=idx, n_cols=k)  # B fits in L2: row order
+    monkeypatch.setattr(_csr.SpmmPlan, "ORDER_ABOVE_COLS", 0)
+    plan = _csr.SpmmPlan(ptr, n_rows, torch.float32, indices=idx, n_cols=k)
+    a, b = (np.stack(p.plan.unit_table(), 1) for p in (plain, plan))
+    nb = plain.plan.n_block_units
+    assert np.array_equal(a[:nb], b[:nb])
+    if skewed:
+        assert np.array_equal(a, b)
+    else:
+        assert np.array_equal(a[np.lexsort(a.T[::-1])], b[np.lexsort(b.T[::-1])])
+        win = host(idx)[b[nb:, 0]].astype(np.int64) * 1024 // k
+        assert (b[nb:, 3] < -1).sum() >= 1024 and np.all(np.diff(win) >= 0)
+    C = [_csr.spmm(data, idx, ptr, n_rows, k, B, p, torch.empty(n_rows, 64, device="cuda")) for p in (plain, plan)]
+    assert torch.equal(C[0], C[1]) and plan.counters_clear()
+
+
 # ---------------------------------------------------------------- opt entry points / API contract
 
 def test_spmm_opt_entry_points_agree():
