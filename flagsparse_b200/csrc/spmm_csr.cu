@@ -590,8 +590,10 @@ __device__ __forceinline__ void acc_shfl_add(WideAcc<DT, V>& a, int m) { a.shfl_
 // the final rounding whatever the row length (the chunk and team partials
 // are combined compensated as well); 3 fp64 sums of the exact products
 // (WideAcc), far inside that bound.  The fp32-accumulated types' rows over
-// kCompensateAbove nonzeros use 3 in column tiles of 512 bytes, 2 in narrower
-// ones (fp64 sums cost 3-5 % on 256-byte rows) and 1 in widths off the slices.
+// kCompensateAbove nonzeros use 3 in column tiles of 512 bytes and in widths off
+// the slices (against mode 1 there, 400,000-row Zipf matrix: fp32, 47 columns 324
+// -> 297 us; bf16, 98 columns 529 -> 436 us), 2 in the other slices (fp64 sums
+// cost 3-5 % on 256-byte rows).
 template <int DT, int MODE, int V>
 struct ChunkAcc;
 template <int DT, int V>
@@ -1004,9 +1006,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     if constexpr (kCompLong<DT, COMP>) {
       if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
         constexpr bool k32 = E * int(sizeof(S)) == 32;
-        if constexpr (!Slice<S, E, P>::kWhole) {
-          chunk(std::integral_constant<int, 1>());
-        } else if constexpr (kOneTeam) {
+        if constexpr (kOneTeam || !Slice<S, E, P>::kWhole) {
           chunk(std::integral_constant<int, 3>());
         } else {
           if (k32 && !FUSED && T == 16) chunk(std::integral_constant<int, k32 && !FUSED ? 3 : 2>());
