@@ -197,6 +197,11 @@ constexpr int kSpmvBatch = 32 * kSpmvItems;
 // Row-block units: kP consecutive nonzeros per lane and pass (one wide load of
 // columns, one or two of values), kCap the largest window: a unit holds <= cap
 // rows, whose local indices fit the end marks' bytes, and < 2*cap nonzeros.
+// A large window fills more of a unit's last pass and spreads its fixed chain of
+// loads over more rows: against 224 for the 2- and 4-byte types and 128 for the
+// wider ones, 252 takes a 1 M-row stencil from 37 to 33 us in fp64 and 26.7 to
+// 22.6 in fp32, Poisson(16) from 39 to 31 us in fp64 (300,000 rows) and 71.8 to
+// 70.3 in fp32 (1 M rows), fp64 Zipf (1 M rows) from 139 to 123 us.
 // Four per lane rather than eight: the next pass's run is held in registers
 // beside the current one, and eight spill at 64 registers (2 M-row Zipf(2)
 // matrix: 94 against 135 us for this launch, 107 us for the product staging
@@ -207,7 +212,7 @@ struct SpmvRow {
   using S = typename VT<DT>::Store;
   static constexpr int kP = sizeof(S) <= 8 ? 4 : 2;
   static constexpr int kPass = 32 * kP;
-  static constexpr int kCap = sizeof(S) <= 4 ? 224 : 128;
+  static constexpr int kCap = 252;
   static constexpr int kMarkBytes = (2 * kCap + 2 * kP + 15) & ~15;
   static_assert(kCap < 255, "local row index + 1 is one byte");
 };

@@ -176,7 +176,7 @@ class NativeSpmvPlan:
         code = nat.dtype_code(dtype)
         device = indptr.device
         self.dtype = dtype
-        self.cap = int(cap) if cap is not None else int(lib.fsb_spmv_default_cap(code))
+        self.cap = int(cap) if cap is not None else int(lib.fsb_spmv_max_cap(code))
         self.chunk_nnz = int(chunk_nnz) if chunk_nnz is not None else int(lib.fsb_spmv_default_chunk(code))
         n_rows = int(n_rows)
         st = nat.stream_of(device)

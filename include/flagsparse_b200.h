@@ -199,8 +199,10 @@ typedef struct fsb_spmv_plan {
  * compensated.  Off by default. */
 #define FSB_SPMV_FAST_SHORT_ROWS 1
 
-/* Row-block window: 224 for f16 / bf16 / f32 (14 nonzeros per lane), 128 for
- * the wider types; any smaller window is accepted. */
+/* Row-block windows: any from 1 to the largest is accepted.  The largest, 252,
+ * measured fastest; the default is 224 for f16 / bf16 / f32, 128 for the wider
+ * types. */
+FSB_API int32_t fsb_spmv_max_cap(int dtype);
 FSB_API int32_t fsb_spmv_default_cap(int dtype);
 /* Long-row chunk: 1024 nonzeros for f16 / bf16 / f32, 512 for the wider types;
  * any positive multiple of 256 is accepted. */

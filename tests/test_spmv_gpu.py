@@ -354,7 +354,7 @@ def test_spmv_row_blocks_run_edges(dname, idx_dt, skip):
     """Row-block passes (runs of 4 or 2 nonzeros per lane): rows that end on, before and after
     the ends of runs and passes, empty rows between and around them, rows at the window, arrays
     that start off the wide loads' boundaries; and one infinite x entry stays in its own rows."""
-    lens = ([0, 1, 0, 2, 3, 4, 5] + [1] * 9 + [63, 64, 65, 0, 127, 128, 129, 0, 0, 223, 224, 225, 1, 0, 31, 33]
+    lens = ([0, 1, 0, 2, 3, 4, 5] + [1] * 9 + [63, 64, 65, 0, 127, 128, 129, 0, 0, 223, 224, 225, 251, 252, 253, 1, 0, 31, 33]
             + [7] * 40 + [0] * 300 + [128, 128, 96, 32, 2] + [0, 3] * 50 + [1])
     ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
     nnz, k = int(ptr[-1]), 700
