@@ -202,8 +202,14 @@ def ptr(t):
     return t.data_ptr() or None
 
 
+# handle of a device's current stream without a torch.cuda.Stream object around it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_of(device):
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
 
 
 def dtype_code(dtype):

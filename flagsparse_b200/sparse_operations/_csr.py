@@ -13,12 +13,14 @@ import torch
 from .. import _native as nat
 
 
-def inspect_csr(indices, indptr, n_rows, nnz):
+def inspect_csr(indices, indptr, n_rows, nnz, plan_for=None):
     """Return a dict with indptr[0], indptr[-1], #decreasing steps, min/max column, max row length.
 
-    One kernel, one device-to-host read.
+    One kernel, one device-to-host read.  ``plan_for=(indptr, cap, chunk_nnz)`` (the row pointers a
+    plan will be built from) also runs that plan's analysis before the read, whose result the dict
+    holds as "plan": valid once the checks on the other entries have passed.
     """
-    out = torch.empty(6, dtype=torch.int64, device=indptr.device)
+    out = torch.empty(10, dtype=torch.int64, device=indptr.device)
     if n_rows + 1 == 0:
         raise ValueError("indptr must have at least one entry")
     lib = nat.lib()
@@ -31,8 +33,12 @@ def inspect_csr(indices, indptr, n_rows, nnz):
         ),
         "fsb_csr_inspect",
     )
+    ws = None
+    if plan_for is not None and n_rows > 0:
+        ws = _analyze_plan(plan_for[0], n_rows, plan_for[1], plan_for[2], out[6:])
     v = out.tolist()
     return {
+        "plan": None if ws is None else (ws, v[6:]),
         "first": v[0],
         "last": v[1],
         "decreasing": v[2],
@@ -40,6 +46,19 @@ def inspect_csr(indices, indptr, n_rows, nnz):
         "max_col": v[4] if nnz > 0 else None,
         "max_row_nnz": v[5] if n_rows > 0 else 0,
     }
+
+
+def _analyze_plan(indptr, n_rows, cap, chunk_nnz, totals):
+    """Launches a plan's analysis into ``totals`` (int64[4] on the device); returns its workspace."""
+    lib = nat.lib()
+    ws_bytes = int(lib.fsb_spmv_plan_workspace_bytes(n_rows))
+    ws = torch.empty(max(ws_bytes, 8), dtype=torch.uint8, device=indptr.device)
+    nat.check(
+        lib.fsb_spmv_plan_analyze(nat.ptr(indptr), nat.is64(indptr), n_rows, cap, chunk_nnz, nat.ptr(ws), ws_bytes,
+                                  nat.ptr(totals), nat.stream_of(indptr.device)),
+        "fsb_spmv_plan_analyze",
+    )
+    return ws
 
 
 def transpose_pattern(indices, indptr, shape, out_index_dtype, out_indptr_dtype):
@@ -171,7 +190,8 @@ class NativeSpmvPlan:
     __slots__ = ("seg_row0", "seg_unit0", "units", "partials", "counters", "cap", "chunk_nnz",
                  "n_segs", "n_units", "n_slots", "n_block_units", "dtype", "flags", "_struct")
 
-    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None, fast_short_rows=False, scratch=True):
+    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None, fast_short_rows=False, scratch=True,
+                 analysis=None):
         lib = nat.lib()
         code = nat.dtype_code(dtype)
         device = indptr.device
@@ -180,16 +200,14 @@ class NativeSpmvPlan:
         self.chunk_nnz = int(chunk_nnz) if chunk_nnz is not None else int(lib.fsb_spmv_default_chunk(code))
         n_rows = int(n_rows)
         st = nat.stream_of(device)
-        ws_bytes = int(lib.fsb_spmv_plan_workspace_bytes(n_rows))
-        ws = torch.empty(max(ws_bytes, 8), dtype=torch.uint8, device=device)
-        totals = torch.zeros(4, dtype=torch.int64, device=device)
-        if n_rows > 0:
-            nat.check(
-                lib.fsb_spmv_plan_analyze(nat.ptr(indptr), nat.is64(indptr), n_rows, self.cap,
-                                          self.chunk_nnz, nat.ptr(ws), ws_bytes, nat.ptr(totals), st),
-                "fsb_spmv_plan_analyze",
-            )
-        self.n_segs, self.n_units, self.n_slots, self.n_block_units = (int(v) for v in totals.tolist())
+        ws, totals = None, (0, 0, 0, 0)
+        if analysis is not None:  # of these row pointers, cap and chunk (inspect_csr's plan_for)
+            ws, totals = analysis
+        elif n_rows > 0:
+            out = torch.empty(4, dtype=torch.int64, device=device)
+            ws = _analyze_plan(indptr, n_rows, self.cap, self.chunk_nnz, out)
+            totals = out.tolist()
+        self.n_segs, self.n_units, self.n_slots, self.n_block_units = (int(v) for v in totals)
         self.seg_row0 = torch.empty(self.n_segs + 1, dtype=torch.int32, device=device)
         self.seg_unit0 = torch.empty(self.n_segs + 1, dtype=torch.int32, device=device)
         # fsb_spmv_unit: int64 nnz_begin, nnz_end; int32 row, tag, n_chunks, slot (32 bytes)
@@ -197,7 +215,7 @@ class NativeSpmvPlan:
         if n_rows > 0:
             nat.check(
                 lib.fsb_spmv_plan_build(nat.ptr(indptr), nat.is64(indptr), n_rows, self.cap,
-                                        self.chunk_nnz, nat.ptr(ws), ws_bytes, nat.ptr(self.seg_row0),
+                                        self.chunk_nnz, nat.ptr(ws), int(ws.numel()), nat.ptr(self.seg_row0),
                                         nat.ptr(self.seg_unit0), nat.ptr(self.units), st),
                 "fsb_spmv_plan_build",
             )
@@ -239,13 +257,13 @@ class SpmmPlan:
     plus long-row scratch sized per dense width N (allocated once per N and
     reused; fsb_spmm_csr leaves the tickets zero after every call)."""
 
-    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None, indices=None, n_cols=0):
-        lib = nat.lib()
-        code = nat.dtype_code(dtype)
+    def __init__(self, indptr, n_rows, dtype, cap=None, chunk_nnz=None, indices=None, n_cols=0, analysis=None):
         self.dtype = dtype
-        cap = int(lib.fsb_spmm_default_cap(code)) if cap is None else int(cap)
-        chunk_nnz = int(lib.fsb_spmm_default_chunk(code)) if chunk_nnz is None else int(chunk_nnz)
-        self.plan = NativeSpmvPlan(indptr, n_rows, dtype, cap=cap, chunk_nnz=chunk_nnz, scratch=False)
+        default_cap, default_chunk = self.shape_of(dtype)
+        cap = default_cap if cap is None else int(cap)
+        chunk_nnz = default_chunk if chunk_nnz is None else int(chunk_nnz)
+        self.plan = NativeSpmvPlan(indptr, n_rows, dtype, cap=cap, chunk_nnz=chunk_nnz, scratch=False,
+                                   analysis=analysis)
         if indices is not None and n_cols > self.ORDER_ABOVE_COLS and self.plan.n_slots > 0:
             self._order_chunks(indices, n_cols)
         self._scratch = {}  # n -> (partials, counters, SpmvPlan struct)
@@ -253,6 +271,12 @@ class SpmmPlan:
     # Chunks are put in column order where a B of the widest column tile (512 bytes)
     # is larger than the 126 MB L2; a smaller B stays there in any order.
     ORDER_ABOVE_COLS = (126 << 20) // 512
+
+    @staticmethod
+    def shape_of(dtype):
+        """(window, chunk) of a plan for this value type."""
+        code = nat.dtype_code(dtype)
+        return int(nat.lib().fsb_spmm_default_cap(code)), int(nat.lib().fsb_spmm_default_chunk(code))
 
     def _order_chunks(self, indices, n_cols):
         lib = nat.lib()
@@ -287,8 +311,8 @@ class SpmmPlan:
                                                         ctypes.byref(tk)), "fsb_spmm_scratch_layout")
             device = self.plan.units.device
             slots = self.plan.n_slots
-            partials = torch.empty(max(slots * pb.value, 16), dtype=torch.uint8, device=device)
-            counters = torch.zeros(max(slots * tk.value, 1), dtype=torch.int32, device=device)
+            partials = torch.empty(slots * pb.value, dtype=torch.uint8, device=device)
+            counters = (torch.zeros if slots else torch.empty)(slots * tk.value, dtype=torch.int32, device=device)
             st = nat.SpmvPlan.from_buffer_copy(self.plan._struct)
             st.partials = nat.ptr(partials)
             st.counters = nat.ptr(counters)

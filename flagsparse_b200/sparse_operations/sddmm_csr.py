@@ -255,13 +255,15 @@ def flagsparse_sddmm_csr(data=None, indices=None, indptr=None, x=None, y=None, s
         if return_meta:
             return out, meta
         return out
-    torch.cuda.synchronize()
-    t0 = time.perf_counter()
+    if return_time:
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
     out_tensor, launch_meta = _run_sddmm_prepared(prepared, x.contiguous(), y.contiguous(),
                                                   data.contiguous() if data is not None else None, alpha, beta, out,
                                                   allow_fallback=allow_fallback)
-    torch.cuda.synchronize()
-    elapsed_ms = (time.perf_counter() - t0) * 1000.0
+    if return_time:
+        torch.cuda.synchronize()
+        elapsed_ms = (time.perf_counter() - t0) * 1000.0
     if return_time and return_meta:
         return out_tensor, elapsed_ms, {"prepare_ms": prepare_ms, **launch_meta}
     if return_time:

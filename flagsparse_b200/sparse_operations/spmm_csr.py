@@ -150,11 +150,13 @@ def _spmm_opt_reference_error(candidate, reference, value_dtype):
 
 # ---------------------------------------------------------------- validation / transpose
 
-def _prepare_spmm_csr_matrix(data, indices, indptr, shape):
+def _prepare_spmm_csr_matrix(data, indices, indptr, shape, plan_analysis=None):
     """Validation with the reference's messages (spmm_csr.py:342-404).
 
     One native inspection pass replaces the reference's chain of ``.item()``
     reductions.  Returns int32 kernel indices and int64 kernel row pointers.
+    ``plan_analysis``: a list that receives the SpMM plan's analysis of these row
+    pointers, read back together with the inspection.
     """
     if len(shape) != 2:
         raise ValueError("shape must be a 2-tuple: (n_rows, n_cols)")
@@ -182,7 +184,9 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape):
     data = data.contiguous()
     indices = indices.contiguous()
     indptr = indptr.contiguous()
-    facts = _csr.inspect_csr(indices, indptr, n_rows, nnz)
+    kernel_indptr = indptr.to(torch.int64)
+    plan_for = None if plan_analysis is None else (kernel_indptr, *_csr.SpmmPlan.shape_of(data.dtype))
+    facts = _csr.inspect_csr(indices, indptr, n_rows, nnz, plan_for)
     if facts["first"] != 0:
         raise ValueError("indptr[0] must be 0")
     if facts["last"] != nnz:
@@ -195,7 +199,8 @@ def _prepare_spmm_csr_matrix(data, indices, indptr, shape):
         if facts["max_col"] > _INDEX_LIMIT_INT32:
             raise ValueError("column indices exceed the int32 range supported by the Triton kernel")
     kernel_indices = indices.to(torch.int32) if indices.dtype == torch.int64 else indices
-    kernel_indptr = indptr.to(torch.int64)
+    if plan_analysis is not None:
+        plan_analysis.append(facts["plan"])
     row_lengths = kernel_indptr[1:] - kernel_indptr[:-1] if n_rows > 0 else kernel_indptr.new_empty((0,))
     return data, kernel_indices, kernel_indptr, n_rows, n_cols, row_lengths, int(facts["max_row_nnz"])
 
@@ -362,8 +367,9 @@ def _native_spmm_into(data, kernel_indices, kernel_indptr, n_rows, n_cols, B, pl
     return _csr.spmm(data, kernel_indices, kernel_indptr, n_rows, n_cols, B, plan, out, compensated=compensated)
 
 
-def _spmm_plan(kernel_indices, kernel_indptr, shape, dtype):
-    return _csr.SpmmPlan(kernel_indptr, int(shape[0]), dtype, indices=kernel_indices, n_cols=int(shape[1]))
+def _spmm_plan(kernel_indices, kernel_indptr, shape, dtype, analysis=None):
+    return _csr.SpmmPlan(kernel_indptr, int(shape[0]), dtype, indices=kernel_indices, n_cols=int(shape[1]),
+                         analysis=analysis)
 
 
 def _row_major_out(out, n_rows, n, dtype, device):
@@ -405,8 +411,9 @@ def flagsparse_spmm_csr(
     if max_segments is not None and max_segments <= 0:
         raise ValueError("max_segments must be positive when provided")
 
+    analysis = None if _spmm_op_transposes(op_code) else []  # A^T's plan is another one
     data, kernel_indices, kernel_indptr, n_rows, n_cols, _rl, max_row_nnz = _prepare_spmm_csr_matrix(
-        data, indices, indptr, shape
+        data, indices, indptr, shape, analysis
     )
     if B.ndim != 2:
         raise ValueError("B must be a 2D dense tensor")
@@ -448,7 +455,8 @@ def flagsparse_spmm_csr(
         torch.cuda.synchronize()
         if _spmm_op_transposes(op_code):
             symbolic_ms = (time.perf_counter() - t0) * 1000.0
-    plan = _spmm_plan(kernel_indices, kernel_indptr, (n_rows, n_cols), data.dtype)
+    plan = _spmm_plan(kernel_indices, kernel_indptr, (n_rows, n_cols), data.dtype,
+                      analysis=analysis[0] if analysis else None)
     if max_segments is not None or block_nnz is not None:
         if max_row_nnz is None:
             max_row_nnz = int((kernel_indptr[1:] - kernel_indptr[:-1]).max().item()) if n_rows > 0 else 0

@@ -272,7 +272,7 @@ def _prepare_spmv_csr_matrix(data, indices, indptr, shape, index_fallback_policy
 
 
 def _validate_spmv_x(x, prepared):
-    if x is None or not torch.is_tensor(x):
+    if not isinstance(x, torch.Tensor):
         raise TypeError("x must be a torch.Tensor")
     if x.ndim != 1:
         raise ValueError("x must be a 1D tensor")
@@ -280,7 +280,7 @@ def _validate_spmv_x(x, prepared):
         raise ValueError("x must be a CUDA tensor")
     if x.dtype != prepared.data.dtype:
         raise TypeError("x dtype must match sparse matrix dtype")
-    if x.numel() != prepared.n_cols:
+    if x.shape[0] != prepared.n_cols:
         raise ValueError(f"x length must be n_cols={prepared.n_cols}, got {x.numel()}")
     if x.device != prepared.data.device:
         raise ValueError("x must be on the same device as sparse matrix data")
@@ -353,24 +353,25 @@ def prepare_spmv_csr(
 
 def _native_spmv_csr_impl_prepared(prepared, x, out=None):
     """One native SpMV launch: y = A x for the prepared (already op-applied) matrix."""
-    y = out if out is not None else torch.empty(prepared.n_rows, dtype=prepared.data.dtype, device=prepared.data.device)
+    data, indices, indptr = prepared.data, prepared.kernel_indices, prepared.kernel_indptr
+    y = out if out is not None else data.new_empty(prepared.n_rows)
     if prepared.n_rows == 0:
         return y
     plan = prepared.native_plan()
     nat.check(
         nat.lib().fsb_spmv_csr(
-            nat.dtype_code(prepared.data.dtype),
-            nat.ptr(prepared.data),
-            nat.ptr(prepared.kernel_indices),
-            nat.is64(prepared.kernel_indices),
-            nat.ptr(prepared.kernel_indptr),
-            nat.is64(prepared.kernel_indptr),
+            nat.dtype_code(data.dtype),
+            nat.ptr(data),
+            nat.ptr(indices),
+            nat.is64(indices),
+            nat.ptr(indptr),
+            nat.is64(indptr),
             prepared.n_rows,
             prepared.n_cols,
             nat.ptr(x),
             nat.ptr(y),
             plan.struct_ref(),
-            nat.stream_of(y.device),
+            nat.stream_of(data.device),
         ),
         "fsb_spmv_csr",
     )
