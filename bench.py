@@ -532,7 +532,7 @@ class SpmmPowerLaw:
         self.ptr = torch.from_numpy(c["indptr"]).to(device)
         g = torch.Generator(device=device).manual_seed(2)
         self.B = torch.randn(self.K, n, device=device, generator=g).to(dt)
-        self.plan = _csr.SpmmPlan(self.ptr, self.M, dt)
+        self.plan = _csr.SpmmPlan(self.ptr, self.M, dt, indices=self.ind, n_cols=self.K)
         self.C = torch.empty(self.M, n, dtype=dt, device=device)
         self.route = fs.prepare_spmm_csr_route(self.vals, self.ind, self.ptr, c["shape"])
         self.B_host = self.B.cpu().pin_memory()

@@ -20,9 +20,8 @@
 //    row adds all partials in a fixed order and resets the ticket, so results
 //    are deterministic.
 //
-// x is gathered with L2-only loads (ld.global.cg): the gathers have no reuse
-// in L1, and where the row-block staging takes most of L1 they run faster
-// without L1 allocation.
+// x is gathered with L2-only loads (ld.global.cg): random gathers have no reuse
+// in L1 (row blocks of a 2 M-row Zipf matrix 94.0 us, 94.4 with plain loads).
 //
 // Replaces _spmv_csr_real_kernel / _spmv_csr_complex_kernel
 // (sparse_operations/spmv_csr.py:179-240) and the bucketed CSR-vector kernels

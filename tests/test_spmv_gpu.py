@@ -349,11 +349,11 @@ def test_spmv_fast_short_rows_mode_within_plain_bound():
 
 @pytest.mark.parametrize("dname", DTYPES)
 @pytest.mark.parametrize("idx_dt", [torch.int32, torch.int64])
-@pytest.mark.parametrize("skip", [0, 1, 6])
-def test_spmv_row_blocks_run_edges(dname, idx_dt, skip):
+@pytest.mark.parametrize("skip,idx_skip", [(0, 0), (1, 1), (6, 6), (3, 0), (0, 2)])
+def test_spmv_row_blocks_run_edges(dname, idx_dt, skip, idx_skip):
     """Row-block passes (runs of 4 or 2 nonzeros per lane): rows that end on, before and after
     the ends of runs and passes, empty rows between and around them, rows at the window, arrays
-    that start off the wide loads' boundaries; and one infinite x entry stays in its own rows."""
+    that start off the wide loads' boundaries, by the same and by different elements; and one infinite x entry stays in its own rows."""
     lens = ([0, 1, 0, 2, 3, 4, 5] + [1] * 9 + [63, 64, 65, 0, 127, 128, 129, 0, 0, 223, 224, 225, 251, 252, 253, 1, 0, 31, 33]
             + [7] * 40 + [0] * 300 + [128, 128, 96, 32, 2] + [0, 3] * 50 + [1])
     ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
@@ -367,7 +367,7 @@ def test_spmv_row_blocks_run_edges(dname, idx_dt, skip):
     x = rng.uniform(-1, 1, k) + (1j * rng.uniform(-1, 1, k) if cplx else 0)
     dt = TORCH_DT[dname]
     d = torch.cat([torch.zeros(skip, dtype=dt, device="cuda"), dev(data, dt)])[skip:]
-    i = torch.cat([torch.zeros(skip, dtype=idx_dt, device="cuda"), dev(idx, idx_dt)])[skip:]
+    i = torch.cat([torch.zeros(idx_skip, dtype=idx_dt, device="cuda"), dev(idx, idx_dt)])[idx_skip:]
     p = fs.prepare_spmv_csr(d, i, dev(ptr), (len(lens), k))
     y = fs.flagsparse_spmv_csr(x=dev(x, dt), prepared=p)
     _check_against_oracle(y, ptr, idx, rounded(data, dname), rounded(x, dname), (len(lens), k), "non", dname, "edges")
