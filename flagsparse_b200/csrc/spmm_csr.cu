@@ -67,27 +67,6 @@ template <> struct RawT<16> { using T = uint4; };
 struct Raw32 { uint32_t r[8]; };
 template <> struct RawT<32> { using T = Raw32; };
 
-// V consecutive elements starting at p; the first nv < V only when the slice
-// crosses column N (the rest read as zero).  ONCE: a streaming (evict-first)
-// load, for data read once that should not displace gathered rows in L2.
-template <typename S, int V, bool ONCE = false>
-__device__ __forceinline__ void load_slice(const S* p, int nv, S (&out)[V]) {
-  if (nv == V) {
-    using Raw = typename RawT<int(sizeof(S)) * V>::T;
-    Raw r = ONCE ? __ldcs(reinterpret_cast<const Raw*>(p)) : __ldg(reinterpret_cast<const Raw*>(p));
-    memcpy(out, &r, sizeof(Raw));
-  } else {
-#pragma unroll
-    for (int j = 0; j < V; ++j) {
-      if (j < nv) {
-        out[j] = p[j];
-      } else {
-        memset(&out[j], 0, sizeof(S));
-      }
-    }
-  }
-}
-
 // A lane's share of a team's column tile: P pieces of E consecutive elements,
 // a team's T lanes side by side in each piece, piece q of lane tl starting at
 // tile column (q * T + tl) * E.  Aligned rows take one 16- or 32-byte piece
@@ -161,23 +140,6 @@ struct Slice {
       }
   }
 };
-
-// Output slices are written once: STREAM makes them streaming (evict-first)
-// stores, so the output does not displace gathered rows in L2.
-template <typename S, int V, bool STREAM = false>
-__device__ __forceinline__ void store_slice(S* p, int nv, const S (&v)[V]) {
-  if (nv == V) {
-    using Raw = typename RawT<int(sizeof(S)) * V>::T;
-    Raw r;
-    memcpy(&r, v, sizeof(Raw));
-    if (STREAM) __stcs(reinterpret_cast<Raw*>(p), r);
-    else *reinterpret_cast<Raw*>(p) = r;
-  } else {
-#pragma unroll
-    for (int j = 0; j < V; ++j)
-      if (j < nv) p[j] = v[j];
-  }
-}
 
 __device__ __forceinline__ __half spmm_store(float v, __half*) { return __float2half_rn(v); }
 __device__ __forceinline__ __nv_bfloat16 spmm_store(float v, __nv_bfloat16*) { return __float2bfloat16_rn(v); }
@@ -1378,7 +1340,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
       __syncwarp();
       for (int k = 0; k < cnt; k += kP * G) {
         S bv[kP][V];
-        R d[kP];
+        [[maybe_unused]] R d[kP];
 #pragma unroll
         for (int q = 0; q < kP; ++q) {
           const int kk = k + q * G + team;
