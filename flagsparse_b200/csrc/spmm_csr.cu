@@ -341,10 +341,13 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // Stages values and columns [s0, s0 + cnt) (cnt <= MAXN) into the warp's
 // shared slices by cp.async, every copy in flight at once; returns the
 // offset of value s0 in sh_a (the values start at sh_a + the offset).  2-byte
-// values move as 4-byte words from the even element at or below s0 (offset 1
-// when s0 is odd; the slice holds MAXN + 2 values); a last value left alone
-// in its word is copied by itself, so nothing past value s0 + cnt - 1 is
-// read.  The caller's __syncwarp() makes the slices visible to all lanes.
+// values move as 4-byte words from the word boundary at or below value s0's
+// address (offset 1 when that is a value earlier: an odd position, or an array
+// that itself starts off a word; the slice holds MAXN + 2 values).  A last value
+// left alone in its word is copied by itself, and so is value 0 of an array
+// that starts inside a word, so nothing before the array or past value
+// s0 + cnt - 1 is read.  The caller's __syncwarp() makes the slices visible to
+// all lanes.
 template <typename S, int MAXN>
 __device__ __forceinline__ int stage_nz(S* sh_a, int32_t* sh_c, const S* __restrict__ data,
                                         const int32_t* __restrict__ col, int64_t s0, int cnt, int lane) {
@@ -352,11 +355,13 @@ __device__ __forceinline__ int stage_nz(S* sh_a, int32_t* sh_c, const S* __restr
   for (int k = lane; k < cnt; k += 32) cp_async<4>(sh_c + k, col + s0 + k);
   if constexpr (sizeof(S) >= 4) {
     for (int k = lane; k < cnt; k += 32) cp_async<int(sizeof(S))>(sh_a + k, data + s0 + k);
-  } else {
-    shift = static_cast<int>(s0 & 1);
-    const S* base = data + (s0 - shift);  // 4-byte aligned (data is)
+  } else if (cnt > 0) {
+    shift = static_cast<int>(reinterpret_cast<uintptr_t>(data + s0) >> 1 & 1);
+    const S* base = data + (s0 - shift);
     const int words = (cnt + shift) >> 1;
-    for (int w = lane; w < words; w += 32) cp_async<4>(sh_a + 2 * w, base + 2 * w);
+    const int alone = s0 < shift ? 1 : 0;  // value 0's word begins before the array
+    for (int w = lane + alone; w < words; w += 32) cp_async<4>(sh_a + 2 * w, base + 2 * w);
+    if (alone && lane == 1) sh_a[1] = ld_once(data);
     if (((cnt + shift) & 1) && lane == 0) sh_a[cnt + shift - 1] = ld_once(data + s0 + cnt - 1);
   }
   cp_async_wait_all();

@@ -10,6 +10,7 @@ import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
 
+import flagsparse_b200 as fs
 from flagsparse_b200 import distributed as fsd
 from flagsparse_b200 import workloads
 from oracle import oracle
@@ -175,6 +176,26 @@ def test_sharded_products_on_one_gpu(world):
     C_scale = oracle.spmm(c["indptr"], c["indices"], np.abs(d), np.abs(B64))
     lens = np.broadcast_to(np.diff(c["indptr"])[:, None], C_ref.shape)
     assert_within(C, C_ref, plain_error_bound("float32", C_ref, C_scale, lens), f"sharded spmm x{world}")
+
+
+@pytest.mark.gpu
+def test_sharded_16_bit_values_on_one_gpu():
+    """Shards of 16-bit values are views that may start off a 4-byte boundary: their products are
+    bitwise those of aligned copies."""
+    c = workloads.zipf_csr(n=20_000, seed=6)
+    data = torch.from_numpy(c["data"]).cuda().to(torch.bfloat16)
+    indices, indptr = torch.from_numpy(c["indices"]).cuda(), torch.from_numpy(c["indptr"]).cuda()
+    x = torch.from_numpy(c["x"]).cuda().to(torch.bfloat16)
+    odd = 0
+    for rank in range(5):
+        sh = fsd.ShardedCsr(data, indices, indptr, c["shape"], rank=rank, world_size=5)
+        odd += sh.data.data_ptr() % 4 == 2
+        p, n = sh.indptr, sh.local_shape
+        assert torch.equal(sh.spmv(x), fs.flagsparse_spmv_csr(sh.data.clone(), sh.indices.clone(), p, x, n))
+        for N in (8, 47, 64):
+            B = torch.randn(c["shape"][1], N, device="cuda").to(torch.bfloat16)
+            assert torch.equal(sh.spmm(B), fs.flagsparse_spmm_csr(sh.data.clone(), sh.indices.clone(), p, B, n))
+    assert odd > 0
 
 
 @pytest.mark.gpu

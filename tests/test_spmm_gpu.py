@@ -530,3 +530,40 @@ def test_spmm_power_law_1m_sampled_rows(dname, N):
                                                B1.abs() + B2.abs())
         lens_t = torch.from_numpy(np.diff(c["indptr"])).cuda().float()[:, None] + 3
         assert bool((diff <= 4 * lens_t * 2.0**-24 * scale_all + 1e-30).all())
+
+
+@pytest.mark.parametrize("dname", ["float16", "bfloat16"])
+@pytest.mark.parametrize("N", [8, 47, 50, 64, 128, 256])
+def test_spmm_values_off_word_boundaries(dname, N):
+    """16-bit values in an array that starts off a 4-byte boundary (a view with an odd offset; NaN
+    around it): forward, fused y, gradients bitwise those of an aligned copy.  Runs that begin with
+    empty rows, with one nonzero, at even and odd positions; chunks of long rows."""
+    lens = np.array([0, 0, 1, 3, 0, 17, 64, 65, 300, 0, 5, 2501, 30, 1, 4800] + [1] * 300 + [2, 9, 0], dtype=np.int64)
+    ptr = np.concatenate([[0], np.cumsum(lens)])
+    k = 5000
+    rng = np.random.Generator(np.random.PCG64(N))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int32)
+    dt = TORCH_DT[dname]
+    aligned = dev(rng.standard_normal(idx.size), dt)
+    wide = torch.full((idx.size + 2,), float("nan"), dtype=dt, device="cuda")
+    wide[1:-1] = aligned
+    i, pt, m = dev(idx), dev(ptr), lens.size
+    B, dY, x = (dev(rng.standard_normal(s), dt) for s in ((k, N), (m, N), k))
+    prep = fs.prepare_spmm_csr_autograd(aligned, i, pt, (m, k))
+    got = []
+    for v in (aligned, wide[1:-1]):
+        plan = _csr.SpmmPlan(pt, m, dt)
+        C = [_csr.spmm(v, i, pt, m, k, B, plan, torch.empty(m, N, dtype=dt, device="cuda"), compensated=c)
+             for c in (False, True)]
+        once = fs.flagsparse_spmm_csr(v, i, pt, B, (m, k))
+        leaf, X = v.detach().requires_grad_(True), B.clone().requires_grad_(True)
+        Y = fs.flagsparse_spmm_csr_autograd(leaf, X, prepared=prep)
+        got.append(C + [once, Y.detach(), *torch.autograd.grad(Y, (leaf, X), dY)])
+        y = torch.empty(m, dtype=dt, device="cuda")
+        if _csr.spmm_spmv(v, i, pt, m, k, B, plan, torch.empty_like(C[0]), x, y):
+            got[-1].append(y)
+    assert wide[1:-1].data_ptr() % 4 == 2 and len(got[0]) == len(got[1])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(host(aligned), dname), (m, k), rounded(host(B), dname), "non")
+    _check(got[1][0], ref, scale, n, dname, f"{dname} N={N}")
