@@ -284,7 +284,7 @@ __device__ __forceinline__ void put_y(double& o, double v) { o = v; }
 // y accumulator of the fused SpMM + SpMV.  For 2- and 4-byte values every
 // product is exact in fp64, so an fp64 sum is at least as accurate as Dot2 in
 // fp32 and costs one DFMA per term; fp64 values keep the Dot2 pair.  A
-// long-row partial takes the two real slots of scratch column n.
+// long-row partial takes the two real slots of its scratch slot's last column.
 template <typename R> struct YAcc;
 template <> struct YAcc<float> {
   double s;
@@ -705,10 +705,13 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
   }
   R* part = static_cast<R*>(plan.partials);
   const int64_t first = int64_t(slot) + (tag + 1);  // slot of the row's first chunk
+  // y's partial takes the slot's last column, which no lane's share reaches, idle
+  // lanes (past column n) included: a fused row is at most 256 bytes, so a team
+  // covers at most 128 columns of the slot's 256
+  [[maybe_unused]] const int64_t yc = pstride - 1;
   if (team == 0) acc.store_partial(part + (int64_t(slot) * pstride + c0) * kER);
   if constexpr (FUSED) {
-    // y's partial sits in the slot's column n (n < pstride for the fused path)
-    if (lane == 0 && tile == 0) yacc.store(part + (int64_t(slot) * pstride + n) * kER);
+    if (lane == 0 && tile == 0) yacc.store(part + (int64_t(slot) * pstride + yc) * kER);
   }
   // the sum of partials from, from + step, ... (count of them) in this order,
   // on every team
@@ -723,7 +726,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
   auto total_y = [&](int64_t from, int64_t step, int count) {
     YAcc<R> fy;
     fy.zero();
-    for (int c = 0; c < count; ++c) fy.add_stored(part + ((from + c * step) * pstride + n) * kER);
+    for (int c = 0; c < count; ++c) fy.add_stored(part + ((from + c * step) * pstride + yc) * kER);
     return fy;
   };
   const ChunkJoin join(nch, -(tag + 1), first);
@@ -732,7 +735,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
     const Acc g = total(join.group_slot, 1, join.group_size);
     if (team == 0) g.store_partial(part + (join.group_slot * pstride + c0) * kER);
     if constexpr (FUSED)
-      if (lane == 0 && tile == 0) total_y(join.group_slot, 1, join.group_size).store(part + (join.group_slot * pstride + n) * kER);
+      if (lane == 0 && tile == 0) total_y(join.group_slot, 1, join.group_size).store(part + (join.group_slot * pstride + yc) * kER);
   }
   if (!join_ticket(plan.counters + first * cps + tile, join.members, lane)) return;
   const Acc fin = total(first, join.step, join.members);
@@ -1526,8 +1529,8 @@ bool spmm_whole_slices(int bytes, int64_t n, const void* B, int64_t ldb, const v
 }
 
 // C = A B and y = A x in one launch: the team kernel with the fused y sums.
-// Real types, narrow aligned rows (the team conditions) and n < the slot
-// stride, so that y's long-row partial has a column of its own.
+// Real types, whole aligned slices and rows of at most 256 bytes, which leave
+// y's long-row partial a column of its own in the scratch slots (team_chunk).
 template <int DT>
 int spmm_spmv_fused(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
                     void* C, int64_t ldc, const void* x, void* y, const fsb_spmv_plan& plan, cudaStream_t st) {
@@ -1536,7 +1539,7 @@ int spmm_spmv_fused(const void* data, const int32_t* idx, const int64_t* ptr, co
   if constexpr (VT<DT>::kComplex) {
     return FSB_ERR_UNSUPPORTED;
   } else {
-    if (!(n * int64_t(sizeof(S)) <= 256 && spmm_whole_slices<S>(16, n, B, ldb, C, ldc) && n < spmm_pstride(n)))
+    if (!(n * int64_t(sizeof(S)) <= 256 && spmm_whole_slices<S>(16, n, B, ldb, C, ldc)))
       return FSB_ERR_UNSUPPORTED;
     if constexpr (kSlice32<DT, false, true>) {
       if (!(plan.flags & FSB_SPMM_COMPENSATED) && n * int64_t(sizeof(S)) >= kSlice32Row<true> &&

@@ -332,7 +332,7 @@ def spmm_spmv(data, indices, indptr, n_rows, n_cols, B, plan, out, x, y, compens
     """out = A @ B and y = A @ x in one launch through fsb_spmm_spmv_csr.
 
     Returns False (nothing launched) when the fused kernel does not apply
-    (complex values, wide or misaligned dense rows, N a multiple of 256).
+    (complex values, wide or misaligned dense rows).
     """
     n = int(B.shape[1])
     rc = nat.lib().fsb_spmm_spmv_csr(

@@ -567,3 +567,32 @@ def test_spmm_values_off_word_boundaries(dname, N):
         assert torch.equal(a, b)
     ref, scale, n = _oracle_spmm(ptr, idx, rounded(host(aligned), dname), (m, k), rounded(host(B), dname), "non")
     _check(got[1][0], ref, scale, n, dname, f"{dname} N={N}")
+
+
+@pytest.mark.parametrize("dname,N", [("float32", 12), ("float32", 20), ("float32", 24), ("float32", 40),
+                                    ("float16", 24), ("bfloat16", 40), ("float64", 6), ("float64", 20)])
+@pytest.mark.parametrize("compensated", [False, True])
+def test_fused_long_rows_with_idle_lanes(dname, N, compensated):
+    """C = A B and y = A x in one launch at widths that leave lanes of a team past the last column
+    (16- and 32-byte slices), on rows of 1 to 200 chunks: both sums against the oracle, the same bits
+    on a second call, tickets left at zero."""
+    lens = np.array([n * 128 + d for n in (1, 2, 15, 16, 17, 18, 32, 33, 48, 49, 200) for d in (0, -1)] + [0, 3, 40])
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    k, m = 26_000, lens.size
+    rng = np.random.Generator(np.random.PCG64(N))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int32)
+    dt = TORCH_DT[dname]
+    data, B, x = rng.standard_normal(idx.size), rng.standard_normal((k, N)), rng.standard_normal(k)
+    d, i, pt, Bd, xd = dev(data, dt), dev(idx), dev(ptr), dev(B, dt), dev(x, dt)
+    plan = _csr.SpmmPlan(pt, m, dt, chunk_nnz=128)
+    out = []
+    for _ in range(2):
+        C, y = torch.empty(m, N, dtype=dt, device="cuda"), torch.empty(m, dtype=dt, device="cuda")
+        assert _csr.spmm_spmv(d, i, pt, m, k, Bd, plan, C, xd, y, compensated)
+        out.append((C, y))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]) and plan.counters_clear()
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(data, dname), (m, k), rounded(B, dname), "non")
+    _check(out[0][0], ref, scale, n, dname, f"{dname} N={N}", compensated)
+    yref = oracle.spmv(ptr, idx, rounded(data, dname), rounded(x, dname))
+    ysc = oracle.spmv_abs(ptr, idx, np.abs(rounded(data, dname)), np.abs(rounded(x, dname)))
+    assert_within(host(out[0][1]).astype(np.float64), yref, spmv_error_bound(dname, yref, ysc, lens), "fused y")
