@@ -205,18 +205,20 @@ constexpr int kSpmvBatch = 32 * kSpmvItems;
 // beside the current one, and eight spill at 64 registers (2 M-row Zipf(2)
 // matrix: 94 against 135 us for this launch, 107 us for the product staging
 // and merge path it replaced; 1 M rows of Poisson(16): 72 against 106 and 84).
-// Two per lane in fp64 measured 41 against 37.5 us on a 1 M-row stencil.
-template <int DT>
+// Two per lane measured slower in fp64 (41 against 37.5 us on a 1 M-row stencil)
+// and in complex fp64 (Poisson(16) on 500,000 rows 115 against 78 us, Poisson(60)
+// on 200,000 rows 187 against 131 us, the stencil 81 against 57 us; the staged
+// kernel took 115, 165 and 82).
 struct SpmvRow {
-  using S = typename VT<DT>::Store;
-  static constexpr int kP = sizeof(S) <= 8 ? 4 : 2;
+  static constexpr int kP = 4;
   static constexpr int kPass = 32 * kP;
   static constexpr int kCap = 252;
   static constexpr int kMarkBytes = (2 * kCap + 2 * kP + 15) & ~15;
   static_assert(kCap < 255, "local row index + 1 is one byte");
+  static_assert(kP == 4, "a run's marks are one 32-bit word");
 };
 
-// N consecutive elements at p (aligned to their size, at most 32 bytes), read
+// N consecutive elements at p (aligned to their size or to 32 bytes), read
 // once: 32-byte loads where there are that many.
 template <typename T, int N>
 __device__ __forceinline__ void ld_run(const T* p, T (&out)[N]) {
@@ -377,7 +379,7 @@ k_spmv_rows(const typename VT<DT>::Store* __restrict__ data, const IT* __restric
             typename VT<DT>::Store* __restrict__ y, const fsb_spmv_unit* __restrict__ units, int64_t n_units,
             int64_t n_rows) {
   using S = typename VT<DT>::Store;
-  using Row = SpmvRow<DT>;
+  using Row = SpmvRow;
   constexpr int kP = Row::kP;
   using Acc = typename std::conditional<(sizeof(S) <= 4), SpmvWide<DT>, SpmvAcc<DT, SHORT_COMP>>::type;
   __shared__ __align__(16) uint8_t sh_mark[kSpmvWarps][Row::kMarkBytes];
@@ -456,10 +458,8 @@ k_spmv_rows(const typename VT<DT>::Store* __restrict__ data, const IT* __restric
         }
         __syncwarp();
       }
-      uint32_t mw[(kP + 3) / 4];
-#pragma unroll
-      for (int w = 0; w < (kP + 3) / 4; ++w) mw[w] = 0;
-      if (p < end) memcpy(mw, __builtin_assume_aligned(mark + p, kP), kP);
+      uint32_t marks = 0;
+      if (p < end) memcpy(&marks, __builtin_assume_aligned(mark + p, kP), kP);
       // sums in order; the first row that ends in the run may have begun before it
       Acc acc, first;
       acc.zero();
@@ -468,7 +468,7 @@ k_spmv_rows(const typename VT<DT>::Store* __restrict__ data, const IT* __restric
 #pragma unroll
       for (int k = 0; k < kP; ++k) {
         acc.add_prod(at[k], xv[k]);
-        const int m = (mw[k / 4] >> (8 * (k % 4))) & 255;
+        const int m = (marks >> (8 * k)) & 255;
         if (m) {
           if (first_row == 0) {
             first = acc;
@@ -563,7 +563,7 @@ template <int DT, typename IT, typename PT>
 static int spmv_launch(const void* data, const void* idx, const void* ptr, const void* x, void* y,
                        int64_t n_rows, const fsb_spmv_plan& plan, cudaStream_t st) {
   // any window up to the type's cap fits a row-block unit's staging (<= cap rows, < 2*cap nonzeros)
-  if (plan.cap < 1 || plan.cap > SpmvRow<DT>::kCap || plan.chunk_nnz % kSpmvBatch != 0) return FSB_ERR_INVALID_ARG;
+  if (plan.cap < 1 || plan.cap > SpmvRow::kCap || plan.chunk_nnz % kSpmvBatch != 0) return FSB_ERR_INVALID_ARG;
   // plain sums of the short rows on request; the 2- and 4-byte types sum them in fp64 at no more cost
   if constexpr (sizeof(typename VT<DT>::Store) > 4)
     if (plan.flags & FSB_SPMV_FAST_SHORT_ROWS)
