@@ -97,6 +97,7 @@ _SIGNATURES = {
         [_c_ptr, _c_int, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr,
          _c_ptr],
     ),
+    "fsb_spmv_best_cap": (_c_i32, [_c_int, _c_i64, _c_i64]),
     "fsb_spmv_max_cap": (_c_i32, [_c_int]),
     "fsb_spmv_default_cap": (_c_i32, [_c_int]),
     "fsb_spmv_default_chunk": (_c_i32, [_c_int]),

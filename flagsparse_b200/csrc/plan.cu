@@ -464,6 +464,25 @@ int32_t fsb_spmv_default_cap(int dtype) { return (dtype == FSB_F16 || dtype == F
 // row indices in one byte (see SpmvRow in spmv_csr.cu).
 int32_t fsb_spmv_max_cap(int dtype) { (void)dtype; return 252; }
 
+// 252 for most matrices (see SpmvRow).  64, which leaves most rows to the
+// long-row kernel, one warp per row with all of its loads in flight, where a
+// row-block warp would walk one or two rows in several dependent passes:
+//  * rows of more than 128 nonzeros on average.  Random columns, us at 252 / 64:
+//    200,000 rows of 150 in f16 159 / 131, fp64 185 / 174, c128 341 / 273;
+//    150,000 rows of 220 in fp32 155 / 135, c64 214 / 174; at a mean of 120 252
+//    is the faster in fp32 (108 / 110) and fp64 (140 / 156);
+//  * rows of more than 64 on average where windows of 252 make less than one
+//    unit per resident warp (148 SMs x 32): 4,000 rows of 100 in bf16 13.7 /
+//    10.3, fp64 10.3 / 8.0; 1,500 rows of 120 10.3 / 6.2.  At a mean of 16 64
+//    is no faster (20,000 rows 8.2 / 8.2), and where the windows fill the chip
+//    252 is (200,000 rows of 80 in fp64 97 / 135).
+int32_t fsb_spmv_best_cap(int dtype, int64_t n_rows, int64_t nnz) {
+  const int32_t widest = fsb_spmv_max_cap(dtype);
+  const bool dense = nnz / 128 > n_rows;
+  const bool few = nnz / 64 > n_rows && nnz + n_rows < int64_t(widest) * 148 * 32;
+  return dense || few ? 64 : widest;
+}
+
 // Long rows are cut into chunks of 256-nonzero batches per warp: four for the
 // 2- and 4-byte real types (fewer tickets on the gather-bound long rows), two
 // for the wider types.

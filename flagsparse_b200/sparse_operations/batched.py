@@ -90,7 +90,8 @@ class BatchedCsr:
         self.B = torch.zeros(self.n_cols, self.n_dense, dtype=dtype, device=device)
         self.y = torch.empty(self.n_rows, dtype=dtype, device=device)
         self.C = torch.empty(self.n_rows, self.n_dense, dtype=dtype, device=device)
-        self.spmv_cfg = {"cap": int(nat.lib().fsb_spmv_max_cap(nat.dtype_code(dtype))), "chunk": 512}
+        cap = int(nat.lib().fsb_spmv_best_cap(nat.dtype_code(dtype), self.n_rows, self.data.numel()))
+        self.spmv_cfg = {"cap": cap, "chunk": 512}
         self.spmm_cfg = dict(SPMM_CANDIDATES[0])
         self._spmv_plan = self._spmm_plan = None
         self._graph = None

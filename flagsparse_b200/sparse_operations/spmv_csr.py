@@ -163,7 +163,8 @@ class PreparedCsrSpmv:
     def native_plan(self):
         """The native unit plan, built on first use and cached."""
         if self._native_plan is None:
-            self._native_plan = _csr.NativeSpmvPlan(self.kernel_indptr, self.n_rows, self.data.dtype)
+            cap = nat.lib().fsb_spmv_best_cap(nat.dtype_code(self.data.dtype), self.n_rows, self.data.numel())
+            self._native_plan = _csr.NativeSpmvPlan(self.kernel_indptr, self.n_rows, self.data.dtype, cap=cap)
         return self._native_plan
 
 

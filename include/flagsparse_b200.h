@@ -200,9 +200,12 @@ typedef struct fsb_spmv_plan {
  * sum in fp64 at no more cost. */
 #define FSB_SPMV_FAST_SHORT_ROWS 1
 
-/* Row-block windows: any from 1 to the largest is accepted.  The largest, 252,
- * measured fastest; the default is 224 for f16 / bf16 / f32, 128 for the wider
- * types. */
+/* Row-block windows: any from 1 to the largest (252) is accepted.
+ * fsb_spmv_best_cap gives the one that measured fastest for a matrix of these
+ * sizes: the largest for most, a small one where the rows are long.
+ * fsb_spmv_default_cap (224 for f16 / bf16 / f32, 128 for the wider types) stays
+ * as it was for callers whose plans were built with it. */
+FSB_API int32_t fsb_spmv_best_cap(int dtype, int64_t n_rows, int64_t nnz);
 FSB_API int32_t fsb_spmv_max_cap(int dtype);
 FSB_API int32_t fsb_spmv_default_cap(int dtype);
 /* Long-row chunk: 1024 nonzeros for f16 / bf16 / f32, 512 for the wider types;

@@ -374,3 +374,26 @@ def test_spmv_row_blocks_run_edges(dname, idx_dt, skip, idx_skip):
     x[-1] = np.inf
     bad = ~np.isfinite(host(fs.flagsparse_spmv_csr(x=dev(x, dt), prepared=p)))
     assert np.array_equal(np.nonzero(bad)[0], [hit])
+
+
+@pytest.mark.parametrize("dname", DTYPES)
+@pytest.mark.parametrize("n,mean,cap", [(300, 64, 252), (300, 66, 64), (1500, 140, 64), (20_000, 70, 252),
+                                       (20_000, 130, 64)])
+def test_spmv_window_rule(dname, n, mean, cap):
+    """Matrices of long rows get plans with a small window, by mean row length and size; rows of
+    1 to 4 * mean nonzeros either way."""
+    rng = np.random.Generator(np.random.PCG64(mean))
+    lens = rng.integers(mean // 2, mean + mean // 2, n)
+    lens[:4] = [0, 1, 4 * mean, 64]
+    lens[4:] += (n * mean - lens.sum()) // (n - 4)
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    k = 3000
+    idx = rng.integers(0, k, ptr[-1]).astype(np.int32)
+    cplx = dname.startswith("complex")
+    data = rng.standard_normal(idx.size) + (1j * rng.standard_normal(idx.size) if cplx else 0)
+    x = rng.standard_normal(k) + (1j * rng.standard_normal(k) if cplx else 0)
+    dt = TORCH_DT[dname]
+    p = fs.prepare_spmv_csr(dev(data, dt), dev(idx), dev(ptr), (n, k))
+    assert p.native_plan().cap == cap
+    y = fs.flagsparse_spmv_csr(x=dev(x, dt), prepared=p)
+    _check_against_oracle(y, ptr, idx, rounded(data, dname), rounded(x, dname), (n, k), "non", dname, "window")
