@@ -31,9 +31,16 @@
 namespace fsb {
 namespace {
 
-// Warps per block.  2 rather than 8: a block's place is free when its last warp
-// ends (64 columns of fp32 on a 500,000-node graph: 311 against 361 us at 8).
+// Warps per block.  Team kernel: 2 rather than 8, since a block's place is free
+// when its last warp ends (64 columns of fp32 on a 500,000-node graph: 311
+// against 361 us at 8).  Generic kernel, Poisson(20) on 200,000 rows: 8 where
+// lanes load single 2- or 4-byte elements (fp32 of 513 columns 1875 against 2315
+// us at 2, of 37 columns with fp64 sums 360 against 402 us), 2 in fp64 (257
+// columns 1992 against 2981 us at 8) and with vectors (bf16 of 128 columns with
+// fp64 sums 491 against 604 us, fp32 of 512 columns 1573 against 1657 us).
 constexpr int kSddmmWarps = 2;
+template <int DT, int V>
+constexpr int kSddmmGenericWarps = DT != FSB_F64 && V == 1 ? 8 : 2;
 constexpr int kSddmmGroup = 4;  // nonzeros reduced together
 // K-rows of at least this many bytes take 32-byte pieces where they can: half
 // the lanes per row and half the instructions per nonzero of 16-byte ones (64
@@ -75,7 +82,7 @@ __device__ __forceinline__ double to_acc64(double v) { return v; }
 // grid: one warp per 32 nonzeros.  ACC64: accumulate in fp64 whatever the
 // value type; OUT64: write fp64 results (only with ACC64).
 template <int DT, int V, bool ACC64, bool OUT64>
-__global__ void __launch_bounds__(kSddmmWarps * 32)
+__global__ void __launch_bounds__(kSddmmGenericWarps<DT, V> * 32)
 k_sddmm_csr(const int32_t* __restrict__ row_ids, const int32_t* __restrict__ col, int64_t nnz,
             const typename VT<DT>::Store* __restrict__ x, int64_t ldx, const typename VT<DT>::Store* __restrict__ y,
             int64_t ldy, int64_t k, const typename VT<DT>::Store* __restrict__ in, double alpha, double beta,
@@ -83,7 +90,7 @@ k_sddmm_csr(const int32_t* __restrict__ row_ids, const int32_t* __restrict__ col
   using S = typename VT<DT>::Store;
   using R = typename std::conditional<ACC64, double, typename VT<DT>::Real>::type;
   const int lane = threadIdx.x & 31;
-  const int64_t base = (int64_t(blockIdx.x) * kSddmmWarps + (threadIdx.x >> 5)) * 32;
+  const int64_t base = (int64_t(blockIdx.x) * kSddmmGenericWarps<DT, V> + (threadIdx.x >> 5)) * 32;
   if (base >= nnz) return;  // whole warp leaves together
   const int cnt = nnz - base < 32 ? static_cast<int>(nnz - base) : 32;
   int my_r = 0, my_c = 0;
@@ -398,9 +405,9 @@ int sddmm_launch_mode(const int32_t* row_ids, const int32_t* col, int64_t nnz, c
                       cudaStream_t st) {
   using S = typename VT<DT>::Store;
   using O = typename std::conditional<OUT64, double, S>::type;
-  const int64_t blocks = ceil_div(ceil_div(nnz, 32), kSddmmWarps);
+  const int64_t blocks = ceil_div(ceil_div(nnz, 32), kSddmmGenericWarps<DT, V>);
   if (blocks > INT32_MAX) return FSB_ERR_UNSUPPORTED;
-  k_sddmm_csr<DT, V, ACC64, OUT64><<<(unsigned)blocks, kSddmmWarps * 32, 0, st>>>(
+  k_sddmm_csr<DT, V, ACC64, OUT64><<<(unsigned)blocks, kSddmmGenericWarps<DT, V> * 32, 0, st>>>(
       row_ids, col, nnz, static_cast<const S*>(x), ldx, static_cast<const S*>(y), ldy, k,
       static_cast<const S*>(in), alpha, beta, static_cast<O*>(out));
   FSB_LAUNCH_CHECK();
