@@ -368,6 +368,44 @@ __device__ __forceinline__ int stage_nz(S* sh_a, int32_t* sh_c, const S* __restr
   return shift;
 }
 
+// The same with values read through perm: value k of the stage is
+// vals[perm[s0 + k]]; sh_p, where given, keeps those positions.  4- and 8-byte
+// values are copied asynchronously too: the only waits are for their positions,
+// which come four at a time (eight spill in the kernels below; through registers
+// the values cost 5 % on fp64 rows of 512 bytes).  2-byte values go through
+// registers, two at a time (four: bf16 backward of 128 columns, 200,000 rows of
+// Poisson(20), 216 against 203 us).
+template <typename S>
+__device__ __forceinline__ void stage_perm(S* sh_a, int32_t* sh_c, int32_t* sh_p, const S* __restrict__ vals,
+                                           const int32_t* __restrict__ perm, const int32_t* __restrict__ col,
+                                           int64_t s0, int cnt, int lane) {
+  for (int k = lane; k < cnt; k += 32) cp_async<4>(sh_c + k, col + s0 + k);
+  constexpr int kU = sizeof(S) >= 4 ? 4 : 2;
+  for (int k0 = lane; k0 < cnt; k0 += 32 * kU) {
+    int32_t q[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + 32 * u < cnt) q[u] = ld_once(perm + s0 + k0 + 32 * u);
+    if constexpr (sizeof(S) >= 4) {
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (k0 + 32 * u < cnt) cp_async<int(sizeof(S))>(sh_a + k0 + 32 * u, vals + q[u]);
+    } else {
+      S v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (k0 + 32 * u < cnt) v[u] = vals[q[u]];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (k0 + 32 * u < cnt) sh_a[k0 + 32 * u] = v[u];
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+      if (k0 + 32 * u < cnt && sh_p) sh_p[k0 + 32 * u] = q[u];
+  }
+  cp_async_wait_all();
+}
+
 // Run-local row offsets off[i] = ptr[r0 + i] - s0 for i <= nr (nr < MAXR),
 // every load issued before the first store.
 template <int MAXR>
@@ -419,6 +457,8 @@ constexpr bool kCompLong = !COMP && (DT == FSB_F16 || DT == FSB_BF16 || DT == FS
 //    last taker adds the partials in chunk order.
 // FUSED: every lane also gathers x[col] beside B's row and sums y = A x for
 // the team's rows (identical sums on the team's lanes; lane 0 writes y).
+// PERM: value q of the matrix is data[perm[q]], as the gradient dX = A^T dY
+// reads A's values; its rows over kCompensateAbove nonzeros sum in fp64.
 // ---------------------------------------------------------------------------
 constexpr int kRowUnits = 4;                            // row-block units per row group
 constexpr int kRowStage = kRowUnits * 2 * kSpmmMaxCap;  // staged nonzeros of a run (< 512)
@@ -446,14 +486,30 @@ constexpr int spmm_team_warp_smem_bytes() {
 // for compensated or fused sums, for 32-byte slices (bf16, 128 columns: 172
 // against 195 us at 2.5 and 2 slices ahead in 242 us at 4) and for three or
 // four pieces per lane (80 against 87 us at 4: 47 columns of fp32, a
-// 170,001-row Chung-Lu graph); 2 for complex fp64 and 32-byte slices of fp64.
-template <int DT, bool COMP, bool FUSED, int E, int P>
+// 170,001-row Chung-Lu graph) and for narrow 16-bit rows whose values come
+// through perm (8 columns 60 against 51 us at 4); 2 for complex fp64 and 32-byte
+// slices of fp64.
+template <int DT, bool COMP, bool FUSED, int KP, int E, int P, bool PERM>
 struct SpmmTeamWarps8 {
   static constexpr bool k8 = DT == FSB_F64 || DT == FSB_C64;
   static constexpr bool k32 = E * int(sizeof(typename VT<DT>::Store)) == 32;
+  static constexpr bool kPerm2 = PERM && KP == kSpmmAhead && sizeof(typename VT<DT>::Store) == 2;
   static constexpr int value =
-      DT == FSB_C128 ? 2 : k32 ? (k8 ? 2 : 3) : (!COMP && !FUSED && P < 3 && !k8) ? 4 : 3;
+      DT == FSB_C128 ? 2 : k32 ? (k8 ? 2 : 3) : (!COMP && !FUSED && P < 3 && !k8 && !kPerm2) ? 4 : 3;
 };
+
+// Stages nonzeros [s0, s0 + cnt), cnt <= kRowStage, and returns the first value's place.
+template <typename S, bool PERM>
+__device__ __forceinline__ const S* stage(S* sh_a, int32_t* sh_c, const S* __restrict__ data,
+                                          const int32_t* __restrict__ perm, const int32_t* __restrict__ col, int64_t s0,
+                                          int cnt, int lane) {
+  if constexpr (PERM) {
+    stage_perm<S>(sh_a, sh_c, nullptr, data, perm, col, s0, cnt, lane);
+    return sh_a;
+  } else {
+    return sh_a + stage_nz<S, kRowStage>(sh_a, sh_c, data, col, s0, cnt, lane);
+  }
+}
 
 template <int DT, bool COMP, int V>
 __device__ __forceinline__ void acc_shfl_add(SpmmAcc<DT, COMP, V>& a, int m) {
@@ -615,7 +671,7 @@ __device__ __forceinline__ bool join_ticket(int32_t* counter, int count, int lan
 // KA B-row slices in flight; the team partials are combined by xor-shuffles
 // over the team index, then the chunk is stored directly (one-chunk rows) or
 // as a slot partial whose ticket's last taker adds the partials in chunk order.
-template <int DT, int MODE, bool FUSED, int KA, int E, int P>
+template <int DT, int MODE, bool FUSED, int KA, int E, int P, bool PERM>
 __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restrict__ data,
                                            const int32_t* __restrict__ col,
                                            const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
@@ -624,8 +680,8 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
                                            const Slice<typename VT<DT>::Store, E, P>& sl, int64_t pstride,
                                            int64_t cps,
                                            const typename VT<DT>::Store* __restrict__ x,
-                                           typename VT<DT>::Store* __restrict__ y, typename VT<DT>::Store* sh_a,
-                                           int32_t* sh_c) {
+                                           typename VT<DT>::Store* __restrict__ y, const int32_t* __restrict__ perm,
+                                           typename VT<DT>::Store* sh_a, int32_t* sh_c) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
   constexpr int V = E * P;
@@ -645,7 +701,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
   for (int64_t b0 = s0; b0 < s1; b0 += kRowStage) {
     const int cnt = static_cast<int>(s1 - b0 < kRowStage ? s1 - b0 : int64_t(kRowStage));
     __syncwarp();
-    const S* sv = sh_a + stage_nz<S, kRowStage>(sh_a, sh_c, data, col, b0, cnt, lane);
+    const S* sv = stage<S, PERM>(sh_a, sh_c, data, perm, col, b0, cnt, lane);
     __syncwarp();
     for (int k = 0; k < cnt; k += KA * G) {
       S bv[KA][V];
@@ -748,13 +804,13 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
     if (lane == 0 && tile == 0) put_y(y[row], total_y(first, join.step, join.members).value());
 }
 
-template <int DT, bool COMP, bool FUSED, int KP, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
-__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, E, P>::value * 8 / kTeamWarps<FUSED>)
+template <int DT, bool COMP, bool FUSED, int KP, int E, int P, bool PERM>
+__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, KP, E, P, PERM>::value * 8 / kTeamWarps<FUSED>)
 k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
             const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
             typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int T, int64_t tiles,
             int64_t pstride, int64_t cps, const typename VT<DT>::Store* __restrict__ x,
-            typename VT<DT>::Store* __restrict__ y) {
+            typename VT<DT>::Store* __restrict__ y, const int32_t* __restrict__ perm) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
   constexpr int V = E * P;
@@ -819,7 +875,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
         const int nr = r1 - r0;
         const int cnt = static_cast<int>(s1 - s0);
         __syncwarp();
-        const S* sv = sh_a + stage_nz<S, kRowStage>(sh_a, sh_c, data, col, s0, cnt, lane);
+        const S* sv = stage<S, PERM>(sh_a, sh_c, data, perm, col, s0, cnt, lane);
         stage_offsets<kRowRows>(sh_off, ptr, r0, nr, s0, lane);
         __syncwarp();
         // empty rows get zero slices (one team each)
@@ -966,8 +1022,8 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     // rows of more than kCompensateAbove nonzeros sum compensated in the
     // fp32-accumulated types, partials and all (see ChunkAcc)
     auto chunk = [&](auto mode) {
-      team_chunk<DT, decltype(mode)::value, FUSED, KP, E, P>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile, sl,
-                                                             pstride, cps, x, y, sh_a, sh_c);
+      team_chunk<DT, decltype(mode)::value, FUSED, KP, E, P, PERM>(data, col, B, ldb, n, C, ldc, plan, ud, T, tile,
+                                                                   sl, pstride, cps, x, y, perm, sh_a, sh_c);
     };
     if constexpr (COMP) {
       chunk(std::integral_constant<int, 1>());
@@ -976,7 +1032,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
     if constexpr (kCompLong<DT, COMP>) {
       if (int64_t(nch) * plan.chunk_nnz > kCompensateAbove) {
         constexpr bool k32 = E * int(sizeof(S)) == 32;
-        if constexpr (kOneTeam || !Slice<S, E, P>::kWhole) {
+        if constexpr (kOneTeam || PERM || !Slice<S, E, P>::kWhole) {
           chunk(std::integral_constant<int, 3>());
         } else {
           if (k32 && !FUSED && T == 16) chunk(std::integral_constant<int, k32 && !FUSED ? 3 : 2>());
@@ -1009,7 +1065,7 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
 // which the row changes.  The dot products of a step reduce across the team by
 // a transpose butterfly (log2 of the step's size halving steps, then plain xor
 // steps) in a fixed order; the lanes left holding a finished product write it.
-// With DV false dvals is not formed (dX only).  X is read with streaming loads
+// (dX alone is k_spmm_team over A^T, see spmm_backward.)  X is read with streaming loads
 // and dX written with streaming stores, which keep more of the gathered dY
 // rows in L2 (measured 0.5 % faster).
 // ---------------------------------------------------------------------------
@@ -1024,33 +1080,6 @@ constexpr int spmm_bwd_park_offset() {
 template <int DT, int V>
 constexpr int spmm_bwd_warp_smem_bytes() {
   return spmm_bwd_park_offset<typename VT<DT>::Store>() + 32 * int(sizeof(SpmmAcc<DT, false, V>));
-}
-
-// Stages values (through perm), columns and positions of nonzeros
-// [s0, s0 + cnt), cnt <= kRowStage.
-template <typename S>
-__device__ __forceinline__ void stage_perm(S* sh_a, int32_t* sh_c, int32_t* sh_p, const S* __restrict__ vals,
-                                           const int32_t* __restrict__ perm, const int32_t* __restrict__ col,
-                                           int64_t s0, int cnt, int lane) {
-  for (int k = lane; k < cnt; k += 32) cp_async<4>(sh_c + k, col + s0 + k);
-  constexpr int kU = 4;
-  for (int k0 = lane; k0 < cnt; k0 += 32 * kU) {
-    int32_t q[kU];
-    S v[kU];
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (k0 + 32 * u < cnt) q[u] = ld_once(perm + s0 + k0 + 32 * u);
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (k0 + 32 * u < cnt) v[u] = vals[q[u]];
-#pragma unroll
-    for (int u = 0; u < kU; ++u)
-      if (k0 + 32 * u < cnt) {
-        sh_p[k0 + 32 * u] = q[u];
-        sh_a[k0 + 32 * u] = v[u];
-      }
-  }
-  cp_async_wait_all();
 }
 
 // Reduces d[0..M) of every lane across the T lanes of its team.  On return the
@@ -1146,7 +1175,7 @@ __device__ __forceinline__ void bwd_put_dots(R (&d)[KA], int base, int stride, i
   }
 }
 
-template <int DT, bool DV, int E>
+template <int DT, int E>
 __global__ void __launch_bounds__(kSpmmWarps * 32, SpmmBwdBlocks<DT, E>::value)
 k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __restrict__ perm,
            const int32_t* __restrict__ col, const int64_t* __restrict__ ptr,
@@ -1252,9 +1281,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
       bool open_start = jb < je && sh_off[cur] < jb;
       int park_row = -1;
       S xa[V], xb[V];
-      if constexpr (DV) {
-        if (jb < je) load_x(int64_t(r0) + cur, xa);
-      }
+      if (jb < je) load_x(int64_t(r0) + cur, xa);
       // every team takes the same number of steps: the butterflies are warp-wide
       for (int t = 0; t < per; t += kP) {
         const int j0 = jb + t;
@@ -1264,17 +1291,15 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
         for (int q = 0; q < kP; ++q)  // past je: some nonzero, loaded and not summed
           sl.load(Bl, static_cast<uint32_t>(sh_c[min(j0 + q, max(je - 1, 0))]), lddy, bv[q]);
         int xrow = -1;
-        if constexpr (DV) {
-          if (next_end < je && next_end < j0 + kP) {  // the row changes in this step
-            xrow = cur + 1;
-            while (sh_off[xrow + 1] == next_end) ++xrow;
-            load_x(int64_t(r0) + xrow, xb);
-          }
+        if (next_end < je && next_end < j0 + kP) {  // the row changes in this step
+          xrow = cur + 1;
+          while (sh_off[xrow + 1] == next_end) ++xrow;
+          load_x(int64_t(r0) + xrow, xb);
         }
 #pragma unroll
         for (int q = 0; q < kP; ++q) {
           const int j = j0 + q;
-          if constexpr (DV) d[q] = R(0);
+          d[q] = R(0);
           if (j < je) {
             if (j == next_end) {  // row cur ended before nonzero j
               if (open_start) {
@@ -1289,16 +1314,14 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
                 ++cur;
                 next_end = sh_off[cur + 1];
               } while (next_end == j);
-              if constexpr (DV) {
-                if (cur == xrow) memcpy(xa, xb, sizeof(xa));
-                else load_x(int64_t(r0) + cur, xa);
-              }
+              if (cur == xrow) memcpy(xa, xb, sizeof(xa));
+              else load_x(int64_t(r0) + cur, xa);
             }
             acc.add(sh_a[j], bv[q]);
-            if constexpr (DV) d[q] = dot(bv[q], xa);
+            d[q] = dot(bv[q], xa);
           }
         }
-        if constexpr (DV) bwd_put_dots<S, R, kP>(d, j0, 1, je, T, tl, sh_p, dvals);
+        bwd_put_dots<S, R, kP>(d, j0, 1, je, T, tl, sh_p, dvals);
       }
       // inclusive segmented scan of the open-ended partials over the teams
       const bool open_end = jb < je && next_end > je;  // row cur goes on in later teams
@@ -1333,7 +1356,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
   const int32_t nch = __ldg(&ud->n_chunks), slot = __ldg(&ud->slot);
   const int64_t c0 = int64_t(tl) * V;  // this lane's place in a slot's partials
   S xs[V];
-  if constexpr (DV) load_x(row, xs);
+  load_x(row, xs);
   // WIDE (rows over kCompensateAbove nonzeros, see kCompLong): fp64 sums of the
   // exact products; else plain sums
   auto run_chunk = [&](auto wide) {
@@ -1348,7 +1371,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
       __syncwarp();
       for (int k = 0; k < cnt; k += kP * G) {
         S bv[kP][V];
-        [[maybe_unused]] R d[kP];
+        R d[kP];
 #pragma unroll
         for (int q = 0; q < kP; ++q) {
           const int kk = k + q * G + team;
@@ -1358,9 +1381,9 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
         for (int q = 0; q < kP; ++q) {
           const int kk = k + q * G + team;
           if (kk < cnt) acc.add(sh_a[kk], bv[q]);
-          if constexpr (DV) d[q] = dot(bv[q], xs);
+          d[q] = dot(bv[q], xs);
         }
-        if constexpr (DV) bwd_put_dots<S, R, kP>(d, k + team, G, cnt, T, tl, sh_p, dvals);
+        bwd_put_dots<S, R, kP>(d, k + team, G, cnt, T, tl, sh_p, dvals);
       }
     }
     for (int m = T; m < 32; m <<= 1) acc_shfl_add(acc, m);  // every team now holds the chunk's sum
@@ -1459,17 +1482,18 @@ inline int spmm_team_tile_bytes(int64_t row_bytes, int32_t hint) {
 // order (tile bytes = T * 16), so the blocks of one tile run together; with
 // FSB_SPMM_PERSISTENT, the resident blocks, whose warps stride over the items
 // in the same order.
-template <int DT, bool COMP, bool FUSED = false, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1>
+template <int DT, bool COMP, bool FUSED = false, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1,
+          bool PERM = false>
 int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
                      void* C, int64_t ldc, const fsb_spmv_plan& plan, int T, int64_t tiles, cudaStream_t st,
-                     const void* x = nullptr, void* y = nullptr) {
+                     const void* x = nullptr, void* y = nullptr, const int32_t* perm = nullptr) {
   using S = typename VT<DT>::Store;
   constexpr bool kAligned = P == 1 && E * int(sizeof(S)) >= 16, k32 = E * int(sizeof(S)) == 32;
   const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kTeamWarps<FUSED>;
   const int wide = (kAligned && !k32 && !FUSED && T == 32) ? 1 : 0;
-  auto kern = k_spmm_team<DT, COMP, FUSED, FUSED && k32 ? kFused32Ahead : kSpmmAhead, E, P>;
+  auto kern = k_spmm_team<DT, COMP, FUSED, FUSED && k32 ? kFused32Ahead : kSpmmAhead, E, P, PERM>;
   if constexpr (kAligned && !k32 && !FUSED)
-    if (wide) kern = k_spmm_team<DT, COMP, FUSED, kOneTeamAhead, E, P>;
+    if (wide) kern = k_spmm_team<DT, COMP, FUSED, kOneTeamAhead, E, P, PERM>;
   if (smem > 48 * 1024) {  // opt in to the larger dynamic shared memory once per kernel and device
     static std::atomic<uint64_t> done[2];
     int dev = 0;
@@ -1515,7 +1539,7 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
   kern<<<(unsigned)blocks, kTeamWarps<FUSED> * 32, smem, st>>>(
       static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), ldb, n,
       static_cast<S*>(C), ldc, plan, T, tiles, spmm_pstride(n), spmm_cps<DT>(n), static_cast<const S*>(x),
-      static_cast<S*>(y));
+      static_cast<S*>(y), perm);
   FSB_LAUNCH_CHECK();
   return FSB_OK;
 }
@@ -1557,10 +1581,15 @@ int spmm_spmv_fused(const void* data, const int32_t* idx, const int64_t* ptr, co
   }
 }
 
-// dX = A^T dY (and dvals = SDDMM(dY, X) on A's pattern when dvals is given) in
-// one launch of k_spmm_bwd.  Real types, 16-byte aligned rows of at most 512
-// bytes whose width n is a multiple of 16 / sizeof(value); plain sums, fp64
-// sums on rows over kCompensateAbove nonzeros for the fp32-accumulated types.
+// dX = A^T dY and dvals = SDDMM(dY, X) on A's pattern in one launch of
+// k_spmm_bwd; without dvals, k_spmm_team over A^T with A's values read through
+// perm, the same sums in the same order.  (The dots' kernel without its dots held
+// the positions and fewer warps for nothing: Poisson(20) on 200,000 rows, fp64 of
+// 64 columns 424 -> 266 us, fp32 of 100 columns 293 -> 239 us, bf16 of 200 290 ->
+// 241 us; 16-bit rows of up to 64 bytes 49 -> 51 us at 8 columns.)  Real types,
+// 16-byte aligned rows of at most 512 bytes whose width n is a multiple of 16 /
+// sizeof(value); plain sums, fp64 sums on rows over kCompensateAbove nonzeros for
+// the fp32-accumulated types.
 template <int DT>
 int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, const int64_t* ptr, const void* dY,
                   int64_t lddy, const void* X, int64_t ldx, int64_t n, void* dX, int64_t lddx, void* dvals,
@@ -1581,18 +1610,15 @@ int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, con
       constexpr int E = decltype(e)::value;
       int T = 1;
       while (int64_t(T) * E < n) T *= 2;
+      if (!dvals)
+        return spmm_launch_team<DT, false, false, E, 1, true>(vals, idx, ptr, dY, lddy, n, dX, lddx, plan, T, 1, st,
+                                                              nullptr, nullptr, perm);
       const int64_t items = ceil_div(plan.n_block_units, kRowUnits) + (plan.n_units - plan.n_block_units);
       const unsigned blocks = (unsigned)ceil_div(items, kSpmmWarps);
       const size_t smem = size_t(spmm_bwd_warp_smem_bytes<DT, E>()) * kSpmmWarps;
-      const S* v = static_cast<const S*>(vals);
-      if (dvals)
-        k_spmm_bwd<DT, true, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
-            v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, static_cast<const S*>(X), ldx,
-            static_cast<S*>(dX), lddx, static_cast<S*>(dvals), plan, T, spmm_pstride(n), spmm_cps<DT>(n));
-      else
-        k_spmm_bwd<DT, false, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
-            v, perm, idx, ptr, static_cast<const S*>(dY), lddy, n, nullptr, 0, static_cast<S*>(dX), lddx, nullptr,
-            plan, T, spmm_pstride(n), spmm_cps<DT>(n));
+      k_spmm_bwd<DT, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
+          static_cast<const S*>(vals), perm, idx, ptr, static_cast<const S*>(dY), lddy, n, static_cast<const S*>(X),
+          ldx, static_cast<S*>(dX), lddx, static_cast<S*>(dvals), plan, T, spmm_pstride(n), spmm_cps<DT>(n));
       FSB_LAUNCH_CHECK();
       return int(FSB_OK);
     };

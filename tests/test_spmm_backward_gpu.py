@@ -175,3 +175,15 @@ def test_backward_row_changes_and_idle_lanes(dname, n):
     assert np.array_equal(~np.isfinite(host(dvals)), own)
     bad = ~np.isfinite(host(dX))
     assert np.array_equal(np.nonzero(bad.any(1))[0], np.sort(indices[own])) and not bad[:, 1:].any()
+
+
+@pytest.mark.parametrize("dname,n", CASES + [("float32", 100), ("float32", 24), ("float64", 34), ("float64", 16),
+                                             ("bfloat16", 200), ("float16", 40)])
+def test_backward_dx_alone_same_bits(dname, n):
+    """dX without dvals (the team kernel over A^T, values through the permutation) has the bits of dX
+    beside dvals, on rows of every kind, and leaves the tickets at zero."""
+    ok, mat, X, dY, dX, _, p = _run(dname, n, seed=5)
+    ok2, _, _, _, alone, none, p2 = _run(dname, n, with_dvals=False, seed=5)
+    assert ok and ok2 and none is None and torch.equal(dX, alone)
+    assert p2.t_plan.n_slots > 0 and p2.t_plan.counters_clear()
+    _check(dname, mat, X, dY, alone, None, n)
