@@ -284,7 +284,7 @@ __device__ __forceinline__ void put_y(double& o, double v) { o = v; }
 // y accumulator of the fused SpMM + SpMV.  For 2- and 4-byte values every
 // product is exact in fp64, so an fp64 sum is at least as accurate as Dot2 in
 // fp32 and costs one DFMA per term; fp64 values keep the Dot2 pair.  A
-// long-row partial takes the two real slots of its scratch slot's last column.
+// long-row partial takes the two real slots of the column after the team's.
 template <typename R> struct YAcc;
 template <> struct YAcc<float> {
   double s;
@@ -761,10 +761,10 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
   }
   R* part = static_cast<R*>(plan.partials);
   const int64_t first = int64_t(slot) + (tag + 1);  // slot of the row's first chunk
-  // y's partial takes the slot's last column, which no lane's share reaches, idle
-  // lanes (past column n) included: a fused row is at most 256 bytes, so a team
-  // covers at most 128 columns of the slot's 256
-  [[maybe_unused]] const int64_t yc = pstride - 1;
+  // y's partial takes the column after the team's, which no lane's share reaches,
+  // idle lanes (past column n) included: a fused row is at most 256 bytes, so a
+  // team covers at most 128 columns of the slot's 256
+  [[maybe_unused]] const int64_t yc = int64_t(T) * V;
   if (team == 0) acc.store_partial(part + (int64_t(slot) * pstride + c0) * kER);
   if constexpr (FUSED) {
     if (lane == 0 && tile == 0) yacc.store(part + (int64_t(slot) * pstride + yc) * kER);

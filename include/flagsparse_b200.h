@@ -346,7 +346,7 @@ FSB_API int fsb_spmm_csr(int dtype, const void* data, const int32_t* indices, co
  * the narrow-row SpMM kernel whose team leaders also sum y, compensated, from
  * x[col] gathered beside B's row.  Real dtypes only; needs n * sizeof(value)
  * <= 256, n a multiple of 16 / sizeof(value), 16-byte aligned B and C with
- * such leading dimensions.  y's long-row partials take the last column of the
+ * such leading dimensions.  y's long-row partials take a column past n of the
  * slot scratch that fsb_spmm_scratch_layout sizes for n.  Returns
  * FSB_ERR_UNSUPPORTED otherwise, with nothing launched; the caller then runs
  * fsb_spmm_csr and fsb_spmv_csr.  plan as for fsb_spmm_csr. */
