@@ -1069,7 +1069,11 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
 // and dX written with streaming stores, which keep more of the gathered dY
 // rows in L2 (measured 0.5 % faster).
 // ---------------------------------------------------------------------------
-constexpr int kBwdAhead = 4;  // dY row slices loaded ahead of the sums
+// dY row slices loaded ahead of the sums: 4, and 8 where one 32-lane team of
+// 16-byte slices has the warp to itself (80 registers; Poisson(20) on 200,000
+// rows, 4 / 8: fp32 of 100 columns 435 / 363 us, bf16 of 200 466 / 398, fp64 of
+// 50 621 / 575)
+constexpr int kBwdAhead = 4, kBwdOneTeamAhead = 8;
 
 // Per-warp slice: staged values, columns, positions in A and run-local row
 // offsets, then (16-byte aligned) one parked accumulator per lane.
@@ -1175,7 +1179,7 @@ __device__ __forceinline__ void bwd_put_dots(R (&d)[KA], int base, int stride, i
   }
 }
 
-template <int DT, int E>
+template <int DT, int E, int KP>
 __global__ void __launch_bounds__(kSpmmWarps * 32, SpmmBwdBlocks<DT, E>::value)
 k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __restrict__ perm,
            const int32_t* __restrict__ col, const int64_t* __restrict__ ptr,
@@ -1185,7 +1189,7 @@ k_spmm_bwd(const typename VT<DT>::Store* __restrict__ vals, const int32_t* __res
            int64_t cps) {
   using S = typename VT<DT>::Store;
   using R = typename VT<DT>::Real;
-  constexpr int V = E, kP = kBwdAhead;
+  constexpr int V = E, kP = KP;
   using Acc = SpmmAcc<DT, false, V>;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1616,7 +1620,10 @@ int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, con
       const int64_t items = ceil_div(plan.n_block_units, kRowUnits) + (plan.n_units - plan.n_block_units);
       const unsigned blocks = (unsigned)ceil_div(items, kSpmmWarps);
       const size_t smem = size_t(spmm_bwd_warp_smem_bytes<DT, E>()) * kSpmmWarps;
-      k_spmm_bwd<DT, E><<<blocks, kSpmmWarps * 32, smem, st>>>(
+      auto kern = k_spmm_bwd<DT, E, kBwdAhead>;
+      if constexpr (E == kVmax)
+        if (T == 32) kern = k_spmm_bwd<DT, E, kBwdOneTeamAhead>;
+      kern<<<blocks, kSpmmWarps * 32, smem, st>>>(
           static_cast<const S*>(vals), perm, idx, ptr, static_cast<const S*>(dY), lddy, n, static_cast<const S*>(X),
           ldx, static_cast<S*>(dX), lddx, static_cast<S*>(dvals), plan, T, spmm_pstride(n), spmm_cps<DT>(n));
       FSB_LAUNCH_CHECK();
