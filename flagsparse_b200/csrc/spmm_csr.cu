@@ -374,7 +374,7 @@ __device__ __forceinline__ int stage_nz(S* sh_a, int32_t* sh_c, const S* __restr
 // which come four at a time (eight spill in the kernels below; through registers
 // the values cost 5 % on fp64 rows of 512 bytes).  2-byte values go through
 // registers, two at a time (four: bf16 backward of 128 columns, 200,000 rows of
-// Poisson(20), 216 against 203 us).
+// Poisson(20), 216 against 203 us), past L1 (201 us).
 template <typename S>
 __device__ __forceinline__ void stage_perm(S* sh_a, int32_t* sh_c, int32_t* sh_p, const S* __restrict__ vals,
                                            const int32_t* __restrict__ perm, const int32_t* __restrict__ col,
@@ -394,7 +394,7 @@ __device__ __forceinline__ void stage_perm(S* sh_a, int32_t* sh_c, int32_t* sh_p
       S v[kU];
 #pragma unroll
       for (int u = 0; u < kU; ++u)
-        if (k0 + 32 * u < cnt) v[u] = vals[q[u]];
+        if (k0 + 32 * u < cnt) v[u] = ld_gather(vals + q[u]);
 #pragma unroll
       for (int u = 0; u < kU; ++u)
         if (k0 + 32 * u < cnt) sh_a[k0 + 32 * u] = v[u];
