@@ -32,10 +32,9 @@ namespace {
 // Warps per block, one work item (or unit) per warp.  Items are uneven, and a
 // block's place is free only when its last warp ends: blocks of 2 warps instead
 // of 8 keep more warps resident (1 M-row power-law matrix, 128 columns: bf16
-// 1.54 -> 1.30 ms, fp32 2.35 -> 2.16 ms; single warps: 1.25 / 2.90 ms).  The
-// fused kernel of the batched step stays at 8: its persistent grid levels the
-// items itself (256 uneven matrices: 1.90 against 2.02 ms).
-constexpr int kSpmmWarps = 2;
+// 1.54 -> 1.30 ms, fp32 2.35 -> 2.16 ms; single warps: 1.25 / 2.90 ms).
+// spmm_block_warps has the exceptions.
+constexpr int kSpmmWarps = 2, kMaxSpmmWarps = 8;
 // Rows of at least this many bytes, made of whole 32-byte slices on 32-byte
 // boundaries, give each lane a 32-byte slice: half the lanes per row, so a warp
 // instruction loads, addresses and tests twice the nonzeros.  At 2 warps per
@@ -52,8 +51,6 @@ template <bool FUSED>
 constexpr int kSlice32Row = FUSED ? 64 : 128;
 template <int DT, bool COMP, bool FUSED>
 constexpr bool kSlice32 = FUSED ? DT == FSB_F32 && !COMP : !VT<DT>::kComplex && (!COMP || DT == FSB_F64);
-template <bool FUSED>
-constexpr int kTeamWarps = FUSED ? 8 : kSpmmWarps;
 constexpr int kSpmmBatch = 128;    // nonzeros staged per batch
 constexpr int kSpmmMaxCap = 64;    // row blocks hold < 2*cap <= kSpmmBatch nonzeros
 // B slices a team loads ahead of its sums: 4; 6 in one-team warps; 2 of 32
@@ -805,7 +802,7 @@ __device__ __forceinline__ void team_chunk(const typename VT<DT>::Store* __restr
 }
 
 template <int DT, bool COMP, bool FUSED, int KP, int E, int P, bool PERM>
-__global__ void __launch_bounds__(kTeamWarps<FUSED> * 32, SpmmTeamWarps8<DT, COMP, FUSED, KP, E, P, PERM>::value * 8 / kTeamWarps<FUSED>)
+__global__ void __launch_bounds__(kMaxSpmmWarps * 32, SpmmTeamWarps8<DT, COMP, FUSED, KP, E, P, PERM>::value * 8 / kMaxSpmmWarps)
 k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __restrict__ col,
             const int64_t* __restrict__ ptr, const typename VT<DT>::Store* __restrict__ B, int64_t ldb, int64_t n,
             typename VT<DT>::Store* __restrict__ C, int64_t ldc, fsb_spmv_plan plan, int T, int64_t tiles,
@@ -833,9 +830,9 @@ k_spmm_team(const typename VT<DT>::Store* __restrict__ data, const int32_t* __re
   const uint32_t n_groups = static_cast<uint32_t>(ceil_div(nb, kRowUnits));
   const uint32_t n_items = n_groups + static_cast<uint32_t>(plan.n_units - nb);
   const uint32_t total = n_items * static_cast<uint32_t>(tiles);
-  const uint32_t nwarps = gridDim.x * kTeamWarps<FUSED>;
+  const uint32_t block_warps = blockDim.x >> 5, nwarps = gridDim.x * block_warps;
 
-  for (uint32_t it = blockIdx.x * kTeamWarps<FUSED> + warp; it < total; it += nwarps) {
+  for (uint32_t it = blockIdx.x * block_warps + warp; it < total; it += nwarps) {
     const uint32_t tile = it / n_items, item = it - tile * n_items;
     Slice<S, E, P> sl;  // pieces past N load column 0 and are not stored
     sl.set(tile, T, tl, n);
@@ -1482,6 +1479,34 @@ inline int spmm_team_tile_bytes(int64_t row_bytes, int32_t hint) {
   return w;
 }
 
+// Warps per block of the team kernel (see kSpmmWarps).  Eight in the fused kernel
+// of the batched step: its persistent grid levels the items itself (256 uneven
+// matrices: 1.90 against 2.02 ms at 2).  More than two also in these 16-byte
+// slices of 8- and 16-byte values, whose rows begin inside 32-byte sectors or
+// take one sector: blocks of two fill the SM's shared memory with warps and leave
+// L1 too small to hold a sector until its other half is read.  Poisson(20) on
+// 200,000 rows, us at 2 / 4 / 8 warps:
+//  * rows of one slice: fp64 45 / 46 / 41;
+//  * narrow tiles of wide rows (tile_bytes): fp64 98 columns 1034 / 1033 / 698,
+//    c64 1002 / 1002 / 702;
+//  * fp64 rows off the 32-byte slices: 98 columns 658 / 659 / 510, Dot2 742 / 746 /
+//    671; 50 columns 263 / 264 / 235, Dot2 334 / 336 / 331 and 505 / 524 / 534 on
+//    Zipf rows; 34 columns 177 / 178 / 203;
+//  * c128 rows of more than one tile off them: 97 columns 1401 / 1293 / 1312, Dot2
+//    1863 / 1881 / 1923; 17 columns 265 / 275 / 278.
+template <int DT, bool COMP, bool FUSED, int E, int P>
+inline int spmm_block_warps(int T, int64_t tiles, int64_t n, int64_t ldb) {
+  constexpr int s = int(sizeof(typename VT<DT>::Store));
+  if constexpr (FUSED) return kMaxSpmmWarps;
+  if constexpr (s == 16) return !COMP && tiles > 1 && (n % 2 != 0 || ldb % 2 != 0) ? 4 : kSpmmWarps;
+  if constexpr (s == 8 && P == 1 && E * s == 16) {
+    const bool narrow = T < 32 && (T == 1 || tiles > 1);
+    const bool off32 = DT == FSB_F64 && T == 32 && (tiles > 1 || (!COMP && n * s > 320));
+    if (narrow || off32) return kMaxSpmmWarps;
+  }
+  return kSpmmWarps;
+}
+
 // The team kernel: one work item per warp, the items of every tile in tile
 // order (tile bytes = T * 16), so the blocks of one tile run together; with
 // FSB_SPMM_PERSISTENT, the resident blocks, whose warps stride over the items
@@ -1493,7 +1518,9 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
                      const void* x = nullptr, void* y = nullptr, const int32_t* perm = nullptr) {
   using S = typename VT<DT>::Store;
   constexpr bool kAligned = P == 1 && E * int(sizeof(S)) >= 16, k32 = E * int(sizeof(S)) == 32;
-  const size_t smem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>()) * kTeamWarps<FUSED>;
+  const int warps = spmm_block_warps<DT, COMP, FUSED, E, P>(T, tiles, n, ldb);
+  constexpr size_t kWarpSmem = size_t(spmm_team_warp_smem_bytes<DT, COMP, E * P>());
+  const size_t smem = kWarpSmem * warps;
   const int wide = (kAligned && !k32 && !FUSED && T == 32) ? 1 : 0;
   auto kern = k_spmm_team<DT, COMP, FUSED, FUSED && k32 ? kFused32Ahead : kSpmmAhead, E, P, PERM>;
   if constexpr (kAligned && !k32 && !FUSED)
@@ -1507,7 +1534,8 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
     }
     const uint64_t bit = uint64_t(1) << (dev & 63);
     if (!(done[wide].load(std::memory_order_acquire) & bit)) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(kWarpSmem * kMaxSpmmWarps)) != cudaSuccess) {
         (void)cudaGetLastError();
         return FSB_ERR_CUDA;
       }
@@ -1516,31 +1544,31 @@ int spmm_launch_team(const void* data, const int32_t* idx, const int64_t* ptr, c
   }
   const int64_t nb = plan.n_block_units;
   const int64_t items = (ceil_div(nb, kRowUnits) + (plan.n_units - nb)) * tiles;
-  int64_t blocks = ceil_div(items, kTeamWarps<FUSED>);  // one work item per warp, tiles in block order
+  int64_t blocks = ceil_div(items, warps);  // one work item per warp, tiles in block order
   if (items >= (int64_t(1) << 32) || blocks > INT32_MAX || (kAligned && ldb > UINT32_MAX)) return FSB_ERR_UNSUPPORTED;
   if (blocks < 1) return FSB_OK;
   if (plan.flags & FSB_SPMM_PERSISTENT) {  // the resident blocks; warps stride over the items
-    static std::atomic<int64_t> resident[2][64];
+    static std::atomic<int64_t> resident[2][kMaxSpmmWarps + 1][64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
       (void)cudaGetLastError();
       return FSB_ERR_CUDA;
     }
-    int64_t r = resident[wide][dev].load(std::memory_order_acquire);
+    int64_t r = resident[wide][warps][dev].load(std::memory_order_acquire);
     if (r == 0) {
       int per_sm = 0, sms = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTeamWarps<FUSED> * 32, smem) != cudaSuccess ||
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem) != cudaSuccess ||
           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm < 1 ||
           sms < 1) {
         (void)cudaGetLastError();
         return FSB_ERR_CUDA;
       }
       r = int64_t(per_sm) * sms;
-      resident[wide][dev].store(r, std::memory_order_release);
+      resident[wide][warps][dev].store(r, std::memory_order_release);
     }
     if (blocks > r) blocks = r;
   }
-  kern<<<(unsigned)blocks, kTeamWarps<FUSED> * 32, smem, st>>>(
+  kern<<<(unsigned)blocks, warps * 32, smem, st>>>(
       static_cast<const S*>(data), idx, ptr, static_cast<const S*>(B), ldb, n,
       static_cast<S*>(C), ldc, plan, T, tiles, spmm_pstride(n), spmm_cps<DT>(n), static_cast<const S*>(x),
       static_cast<S*>(y), perm);
