@@ -1483,26 +1483,32 @@ inline int spmm_team_tile_bytes(int64_t row_bytes, int32_t hint) {
 // of the batched step: its persistent grid levels the items itself (256 uneven
 // matrices: 1.90 against 2.02 ms at 2).  More than two also in these 16-byte
 // slices of 8- and 16-byte values, whose rows begin inside 32-byte sectors or
-// take one sector: blocks of two fill the SM's shared memory with warps and leave
-// L1 too small to hold a sector until its other half is read.  Poisson(20) on
-// 200,000 rows, us at 2 / 4 / 8 warps:
-//  * rows of one slice: fp64 45 / 46 / 41;
-//  * narrow tiles of wide rows (tile_bytes): fp64 98 columns 1034 / 1033 / 698,
-//    c64 1002 / 1002 / 702;
-//  * fp64 rows off the 32-byte slices: 98 columns 658 / 659 / 510, Dot2 742 / 746 /
-//    671; 50 columns 263 / 264 / 235, Dot2 334 / 336 / 331 and 505 / 524 / 534 on
-//    Zipf rows; 34 columns 177 / 178 / 203;
-//  * c128 rows of more than one tile off them: 97 columns 1401 / 1293 / 1312, Dot2
-//    1863 / 1881 / 1923; 17 columns 265 / 275 / 278.
+// take one or two: blocks of two fill the SM's shared memory with warps and leave
+// L1 too small to hold a sector until its other half is read.  us at 2 / 4 / 8
+// warps; Poisson(20) on 200,000 rows, or Poisson(8) on 1 M rows (*):
+//  * fp64 but for rows of 96 bytes: 2 columns 45 / 46 / 41, 8 columns 187 / 188 /
+//    133 *, 14 columns 351 / 352 / 233 *, 98 columns 658 / 659 / 510, Dot2 742 / 746
+//    / 671; 12 columns 64 / 64 / 72 and 201 / 204 / 219 *.  In between two can be
+//    the faster while B is in L2 (34 columns 177 / 178 / 203, 10 columns 62 / 62 /
+//    68 but 269 / 271 / 204 *);
+//  * c64 rows under 128 bytes: 2 columns 45 / 45 / 41, 8 columns 184 / 184 / 135 *;
+//    24 columns 108 / 109 / 119;
+//  * narrow tiles of wide rows (tile_bytes): fp64 98 columns 1034 / 1033 / 698, c64
+//    1002 / 1002 / 702;
+//  * c128 rows of one or two slices: 2 columns 145 / 123 / 128 *; and of more than
+//    one tile off the sectors: 97 columns 1401 / 1293 / 1312; Dot2 1863 / 1881 /
+//    1923, 8 columns 285 / 301 / 307 *.
 template <int DT, bool COMP, bool FUSED, int E, int P>
 inline int spmm_block_warps(int T, int64_t tiles, int64_t n, int64_t ldb) {
   constexpr int s = int(sizeof(typename VT<DT>::Store));
   if constexpr (FUSED) return kMaxSpmmWarps;
-  if constexpr (s == 16) return !COMP && tiles > 1 && (n % 2 != 0 || ldb % 2 != 0) ? 4 : kSpmmWarps;
+  if constexpr (s == 16) {
+    const bool off = tiles > 1 && (n % 2 != 0 || ldb % 2 != 0);
+    return !COMP && (n <= 2 || off) ? 4 : kSpmmWarps;
+  }
   if constexpr (s == 8 && P == 1 && E * s == 16) {
-    const bool narrow = T < 32 && (T == 1 || tiles > 1);
-    const bool off32 = DT == FSB_F64 && T == 32 && (tiles > 1 || (!COMP && n * s > 320));
-    if (narrow || off32) return kMaxSpmmWarps;
+    const bool tiled = tiles > 1 && T < 32;
+    if (tiled || (DT == FSB_F64 ? n * s != 96 : n * s < 128)) return kMaxSpmmWarps;
   }
   return kSpmmWarps;
 }
