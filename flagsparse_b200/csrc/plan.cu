@@ -187,7 +187,11 @@ static int spmv_plan_build_impl(const PT* ptr, int64_t n_rows, int64_t cap, int6
 // chunks keep their order: a graph's hub columns would be hit by every warp at
 // once (bf16 training step on a 500,000-node Chung-Lu graph, 128 columns: 1086 ->
 // 1150 us).  On a 1 M-row power-law matrix, 128 columns: fp32 2.17 -> 1.94 ms,
-// bf16 1.32 -> 1.25 ms.
+// bf16 1.32 -> 1.25 ms.  The plan does not know the width of the products: with a
+// B that stays in L2 the order makes no difference (the same matrix, fp32: 8
+// columns 276.7 / 276.8 us, 16 columns 381 -> 357; 280,000 rows, bf16, 128 columns
+// 252 / 253).  Columns drawn as u^1.5 instead of u, u uniform, still gain (fp32
+// 128 columns 2066 -> 1795 us); as u^2 the order is left alone.
 // ---------------------------------------------------------------------------
 constexpr int kOrderWindows = 1024;
 
@@ -458,6 +462,8 @@ int fsb_csr_inspect(const void* indices, int idx_is_64, const void* indptr, int 
                    : inspect_impl<int32_t, int32_t>(indices, indptr, n_rows, nnz, d_out, st);
 }
 
+// Not the fastest for any matrix (fsb_spmv_best_cap): unchanged for callers whose
+// plans were built with it.
 int32_t fsb_spmv_default_cap(int dtype) { return (dtype == FSB_F16 || dtype == FSB_BF16 || dtype == FSB_F32) ? 224 : 128; }
 
 // A row-block unit holds <= cap rows and < 2*cap nonzeros; 252 keeps its local

@@ -11,11 +11,11 @@
 // 20).  Consecutive nonzeros mostly share a row, so the x slice is an L1 hit.
 //
 // That generic kernel serves every shape; K-rows of up to 1,024 bytes in whole
-// pieces (sddmm_try_team) take the team kernel below, several nonzeros per warp
-// instruction, which keeps the x row per team.  (Narrow rows left most lanes of
-// the generic kernel idle, and rows off the 16-byte slices ran it too: fp32 on
-// a 300,000-node graph, 8 columns 342 -> 42 us, 16 columns 340 -> 60 us, 37
-// columns 416 -> 158 us.)
+// pieces of 8 bytes or more (512 bytes in pieces of 4, 256 of 2: sddmm_try_team)
+// take the team kernel below, several nonzeros per warp instruction, which keeps
+// the x row per team.  (Narrow rows left most lanes of the generic kernel idle,
+// and rows off the 16-byte slices ran it too: fp32 on a 300,000-node graph, 8
+// columns 342 -> 42 us, 16 columns 340 -> 60 us, 37 columns 416 -> 158 us.)
 //
 // Accumulation: fp32 for half / bfloat16 / fp32, fp64 for fp64 (fp64 for every
 // type with FSB_SDDMM_ACC64, which the reference's "acc64" variants select),
@@ -363,10 +363,11 @@ int sddmm_launch_pieces(int pieces, const int32_t* row_ids, const int32_t* col, 
   return sddmm_launch_team<DT, T, E, P>(row_ids, col, nnz, x, ldx, y, ldy, k, in, alpha, beta, out, st);
 }
 
-// The team kernel where a K-row is at most 1,024 bytes of whole pieces: returns
-// 1 when it launched (rc set).  Pieces are the widest of 32 (rows of at least
-// kSlice32 bytes), 16, 8, 4 and 2 bytes that divide K, the leading dimensions
-// and the addresses.
+// The team kernel where 32 lanes hold a K-row: returns 1 when it launched (rc
+// set).  Pieces are the widest of 32 (rows of at least kSlice32 bytes), 16, 8, 4
+// and 2 bytes that divide K, the leading dimensions and the addresses; a lane
+// holds 32 bytes of a row at most (four pieces of 8, two of 16), and four pieces
+// of 4 or 2, so rows of up to 1,024, 512 and 256 bytes.
 template <int DT>
 int sddmm_try_team(const int32_t* row_ids, const int32_t* col, int64_t nnz, const void* x, int64_t ldx,
                    const void* y, int64_t ldy, int64_t k, const void* in, double alpha, double beta, void* out,

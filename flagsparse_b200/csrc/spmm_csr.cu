@@ -51,7 +51,7 @@ template <bool FUSED>
 constexpr int kSlice32Row = FUSED ? 64 : 128;
 template <int DT, bool COMP, bool FUSED>
 constexpr bool kSlice32 = FUSED ? DT == FSB_F32 && !COMP : !VT<DT>::kComplex && (!COMP || DT == FSB_F64);
-constexpr int kSpmmBatch = 128;    // nonzeros staged per batch
+constexpr int kSpmmBatch = 128;    // chunks of long rows are whole multiples of it
 constexpr int kSpmmMaxCap = 64;    // row blocks hold < 2*cap <= kSpmmBatch nonzeros
 // B slices a team loads ahead of its sums: 4; 6 in one-team warps; 2 of 32
 // bytes in the fused kernel, whose x gathers and y sums need the registers
@@ -433,7 +433,8 @@ constexpr bool kCompLong = !COMP && (DT == FSB_F16 || DT == FSB_BF16 || DT == FS
 
 // ---------------------------------------------------------------------------
 // The team kernel.  Teams of T lanes (1 to 32) own a column tile, G = 32 / T
-// teams per warp: T * 16 bytes of aligned rows, T * P pieces of others (Slice).
+// teams per warp: T slices of 16 or 32 bytes of aligned rows, T * P pieces of
+// others (Slice).
 // Rows wider than the tile run as several column tiles; the tile is the
 // slowest work dimension, so while one tile is in flight only that tile's
 // slice of B is being gathered, and a slice that fits in L2 is read from HBM
@@ -443,9 +444,9 @@ constexpr bool kCompLong = !COMP && (DT == FSB_F16 || DT == FSB_BF16 || DT == FS
 // An item is either
 //  * a row group: up to kRowUnits consecutive row-block units, split into runs
 //    of adjacent rows.  A run (<= 256 rows, < 512 nonzeros) is staged in the
-//    warp's shared memory and cut by a merge path over its list of row ends
-//    and nonzeros: every team walks the same number of positions whatever the
-//    row lengths, summing nonzeros and writing a row at its end.  A row that
+//    warp's shared memory and every team takes an equal share of its nonzeros,
+//    whatever the row lengths: it finds its first row by a binary search of the
+//    row offsets, sums nonzeros and writes a row at its end.  A row that
 //    spans teams is finished by a segmented scan over the teams' partial sums
 //    (keys: row indices) in team order;
 //  * a long-row chunk: team g takes nonzeros g, g+G, ...; the team partials
@@ -1514,7 +1515,7 @@ inline int spmm_block_warps(int T, int64_t tiles, int64_t n, int64_t ldb) {
 }
 
 // The team kernel: one work item per warp, the items of every tile in tile
-// order (tile bytes = T * 16), so the blocks of one tile run together; with
+// order (tiles of T slices), so the blocks of one tile run together; with
 // FSB_SPMM_PERSISTENT, the resident blocks, whose warps stride over the items
 // in the same order.
 template <int DT, bool COMP, bool FUSED = false, int E = 16 / int(sizeof(typename VT<DT>::Store)), int P = 1,
@@ -1637,7 +1638,6 @@ int spmm_backward(const void* vals, const int32_t* perm, const int32_t* idx, con
   if constexpr (VT<DT>::kComplex) {
     return FSB_ERR_UNSUPPORTED;
   } else {
-    auto a16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     auto whole = [&](int bytes) {
       return spmm_whole_slices<S>(bytes, n, dY, lddy, dX, lddx) &&
              (!dvals || (ldx * int64_t(sizeof(S)) % bytes == 0 && reinterpret_cast<uintptr_t>(X) % bytes == 0));
@@ -1698,7 +1698,7 @@ int spmm_launch_pieces(const void* data, const int32_t* idx, const int64_t* ptr,
 
 template <int DT, bool COMP>
 int spmm_dispatch(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
-                  int64_t n_cols, void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
+                  void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
   using S = typename VT<DT>::Store;
   constexpr int kVmax = 16 / int(sizeof(S));
   // rows of whole, aligned slices: teams of T lanes over column tiles of T
@@ -1732,10 +1732,10 @@ int spmm_dispatch(const void* data, const int32_t* idx, const int64_t* ptr, cons
 
 template <int DT>
 int spmm_mode(const void* data, const int32_t* idx, const int64_t* ptr, const void* B, int64_t ldb, int64_t n,
-              int64_t n_cols, void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
+              void* C, int64_t ldc, const fsb_spmv_plan& plan, cudaStream_t st) {
   if (plan.flags & FSB_SPMM_COMPENSATED)
-    return spmm_dispatch<DT, true>(data, idx, ptr, B, ldb, n, n_cols, C, ldc, plan, st);
-  return spmm_dispatch<DT, false>(data, idx, ptr, B, ldb, n, n_cols, C, ldc, plan, st);
+    return spmm_dispatch<DT, true>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
+  return spmm_dispatch<DT, false>(data, idx, ptr, B, ldb, n, C, ldc, plan, st);
 }
 
 }  // namespace
@@ -1772,12 +1772,12 @@ int fsb_spmm_csr(int dtype, const void* data, const int32_t* indices, const int6
   if (plan->n_units >= INT32_MAX) return FSB_ERR_UNSUPPORTED;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (dtype) {
-    case FSB_F16: return spmm_mode<FSB_F16>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
-    case FSB_BF16: return spmm_mode<FSB_BF16>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
-    case FSB_F32: return spmm_mode<FSB_F32>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
-    case FSB_F64: return spmm_mode<FSB_F64>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
-    case FSB_C64: return spmm_mode<FSB_C64>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
-    case FSB_C128: return spmm_mode<FSB_C128>(data, indices, indptr, B, ldb, n, n_cols, C, ldc, *plan, st);
+    case FSB_F16: return spmm_mode<FSB_F16>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
+    case FSB_BF16: return spmm_mode<FSB_BF16>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
+    case FSB_F32: return spmm_mode<FSB_F32>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
+    case FSB_F64: return spmm_mode<FSB_F64>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
+    case FSB_C64: return spmm_mode<FSB_C64>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
+    case FSB_C128: return spmm_mode<FSB_C128>(data, indices, indptr, B, ldb, n, C, ldc, *plan, st);
     default: return FSB_ERR_UNSUPPORTED;
   }
 }

@@ -189,7 +189,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 ld_x<__nv_bfloat16>(const _
   return __ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short*>(p)));
 }
 
-constexpr int kSpmvWarps = 8;     // warps per block; one unit per warp
+constexpr int kSpmvWarps = 8;     // warps per block; a unit at a time per warp
 constexpr int kSpmvItems = 8;     // nonzeros per lane per long-row batch
 constexpr int kSpmvBatch = 32 * kSpmvItems;
 
@@ -268,7 +268,7 @@ template <int DT>
 struct SpmvRowMinBlocks { static constexpr int value = (DT == FSB_C128) ? 2 : 4; };
 template <int DT>
 struct SpmvMinBlocks { static constexpr int value = (DT == FSB_C128) ? 2 : (DT == FSB_F64 || DT == FSB_C64) ? 3 : 4; };
-// The long-row kernel keeps fewer values live (no staging, columns one batch
+// The long-row kernel keeps fewer values live (no pass ahead, columns one batch
 // ahead): the 2- and 4-byte real types with 32-bit columns fit 5 blocks per SM
 // without spills.
 template <int DT, typename IT>
@@ -562,7 +562,7 @@ static int spmv_launch_mode(const void* data, const void* idx, const void* ptr, 
 template <int DT, typename IT, typename PT>
 static int spmv_launch(const void* data, const void* idx, const void* ptr, const void* x, void* y,
                        int64_t n_rows, const fsb_spmv_plan& plan, cudaStream_t st) {
-  // any window up to the type's cap fits a row-block unit's staging (<= cap rows, < 2*cap nonzeros)
+  // any window up to kCap fits the end marks (<= cap rows, < 2*cap nonzeros)
   if (plan.cap < 1 || plan.cap > SpmvRow::kCap || plan.chunk_nnz % kSpmvBatch != 0) return FSB_ERR_INVALID_ARG;
   // plain sums of the short rows on request; the 2- and 4-byte types sum them in fp64 at no more cost
   if constexpr (sizeof(typename VT<DT>::Store) > 4)
