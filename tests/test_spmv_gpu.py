@@ -351,7 +351,7 @@ def test_spmv_fast_short_rows_mode_within_plain_bound():
 @pytest.mark.parametrize("idx_dt", [torch.int32, torch.int64])
 @pytest.mark.parametrize("skip,idx_skip", [(0, 0), (1, 1), (6, 6), (3, 0), (0, 2)])
 def test_spmv_row_blocks_run_edges(dname, idx_dt, skip, idx_skip):
-    """Row-block passes (runs of 4 or 2 nonzeros per lane): rows that end on, before and after
+    """Row-block passes (runs of 4 nonzeros per lane): rows that end on, before and after
     the ends of runs and passes, empty rows between and around them, rows at the window, arrays
     that start off the wide loads' boundaries, by the same and by different elements; and one infinite x entry stays in its own rows."""
     lens = ([0, 1, 0, 2, 3, 4, 5] + [1] * 9 + [63, 64, 65, 0, 127, 128, 129, 0, 0, 223, 224, 225, 251, 252, 253, 1, 0, 31, 33]
