@@ -187,3 +187,14 @@ def test_backward_dx_alone_same_bits(dname, n):
     assert ok and ok2 and none is None and torch.equal(dX, alone)
     assert p2.t_plan.n_slots > 0 and p2.t_plan.counters_clear()
     _check(dname, mat, X, dY, alone, None, n)
+
+
+@pytest.mark.parametrize("dname,n", [("float32", 68), ("float32", 100), ("float32", 124), ("float64", 34),
+                                    ("float64", 62), ("bfloat16", 136), ("bfloat16", 248), ("float16", 200)])
+def test_backward_one_team_rows(dname, n):
+    """Rows of 16-byte slices off the 32-byte ones that one 32-lane team walks, eight dY slices ahead,
+    lanes past the last column: dX and dvals against the oracle, tickets at zero."""
+    ok, mat, X, dY, dX, dvals, p = _run(dname, n, seed=3)
+    assert ok
+    _check(dname, mat, X, dY, dX, dvals, n)
+    assert p.t_plan.counters_clear()

@@ -596,3 +596,35 @@ def test_fused_long_rows_with_idle_lanes(dname, N, compensated):
     yref = oracle.spmv(ptr, idx, rounded(data, dname), rounded(x, dname))
     ysc = oracle.spmv_abs(ptr, idx, np.abs(rounded(data, dname)), np.abs(rounded(x, dname)))
     assert_within(host(out[0][1]).astype(np.float64), yref, spmv_error_bound(dname, yref, ysc, lens), "fused y")
+
+
+@pytest.mark.parametrize("dname,N", [("float64", 2), ("float64", 8), ("float64", 12), ("float64", 14), ("float64", 34),
+                                    ("float64", 66), ("complex64", 2), ("complex64", 14), ("complex64", 16),
+                                    ("complex64", 66), ("complex128", 2), ("complex128", 3), ("complex128", 33),
+                                    ("complex128", 64)])
+@pytest.mark.parametrize("items", [1, 9, 70])
+def test_spmm_block_sizes(dname, N, items):
+    """8- and 16-byte values on both sides of the lines between blocks of 2, 4 and 8 warps, from one
+    work item (a block mostly without work) to several blocks: whole rows and 64-byte
+    column tiles against the oracle, and the same bits on the persistent grid."""
+    lens = np.array(([300, 0, 1, 900] + [60, 3, 0, 5] * 2)[:max(1, min(items, 12))] + [7] * (8 * max(0, items - 9)))
+    ptr = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    k, m = 1000, lens.size
+    rng = np.random.Generator(np.random.PCG64(N))
+    idx = np.concatenate([np.sort(rng.choice(k, n, replace=False)) for n in lens]).astype(np.int32)
+    cplx = dname.startswith("complex")
+    draw = lambda *shape: rng.standard_normal(shape) + (1j * rng.standard_normal(shape) if cplx else 0)
+    data, B = draw(idx.size), draw(k, N)
+    dt = TORCH_DT[dname]
+    d, i, pt, Bd = dev(data, dt), dev(idx), dev(ptr), dev(B, dt)
+    plan = _csr.SpmmPlan(pt, m, dt)
+    ref, scale, n = _oracle_spmm(ptr, idx, rounded(data, dname), (m, k), rounded(B, dname), "non")
+    for comp in (False, True):
+        C = [_csr.spmm(d, i, pt, m, k, Bd, plan, torch.empty(m, N, dtype=dt, device="cuda"), compensated=comp, **kw)
+             for kw in ({}, {"persistent": True}, {"tile_bytes": 64}, {"tile_bytes": 64, "persistent": True})]
+        # the oracle rounds the four real products of a complex one before it adds them, an error of
+        # up to 3 u sum |a||b|: beyond the compensated bound, within the plain one
+        _check(C[0], ref, scale, n, dname, f"{dname} N={N}", comp and not cplx)
+        _check(C[2], ref, scale, n, dname, f"{dname} N={N} tiles", comp and not cplx)
+        assert torch.equal(C[0], C[1]) and torch.equal(C[2], C[3])
+        assert plan.counters_clear()
